@@ -127,7 +127,7 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
   double* C = reinterpret_cast<double*>(w);
   w += align256((size_t)batch * Pw::NOUT * nc * 8);
   void* dscratch = w;
-  const long nlm = n_coeff(p->lmax) * batch;
+  const long nlm = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
   derive_cols_kernel<Derive><<<blocks_for(nlm, 128), 128, 0, st>>>(p->lmax, batch, nc, V, d);
   AE_LAUNCH("derive_cols_kernel");
   int s = points_synth(p, V, Gr, batch * Pw::NIN, dscratch, st);
@@ -170,7 +170,7 @@ int run_synth_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, in
   double* Gr = reinterpret_cast<double*>(w);
   w += align256((size_t)batch * Pw::NIN * np * 8);
   void* dscratch = w;
-  const long nlm = n_coeff(p->lmax) * batch;
+  const long nlm = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
   derive_cols_kernel<Derive><<<blocks_for(nlm, 128), 128, 0, st>>>(p->lmax, batch, nc, V, d);
   AE_LAUNCH("derive_cols_kernel");
   const bool direct = Pw::kIdentity && out_b == np;

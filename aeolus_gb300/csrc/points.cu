@@ -63,19 +63,58 @@ int build_points_basis(aeolus_plan_impl* p, const double* lat, const double* lon
   return s;
 }
 
+// Passes of equal width: ceil(N / 8) passes of NT = ceil(N / passes) columns
+// each waste fewer than one column per pass.
+namespace {
+
+template <int NT>
+void synth_pass(long M, int K, int N, const double* B, const double* V, double* out, cudaStream_t st) {
+  const long grid = (M + kPtRows - 1) / kPtRows * ((N + NT - 1) / NT);
+  points_synth_kernel<NT><<<(unsigned)grid, kPtThreads, 0, st>>>(M, K, N, B, V, out);
+}
+
+// Four basis columns per CTA share each point's data values once there are
+// enough columns to fill the chip that way (four CTAs on each SM); one per
+// CTA below that.
+template <int NT>
+void analysis_pass(int M, long K, int N, const double* B, const double* W, double* C, int sm_count, cudaStream_t st) {
+  const long passes = (N + NT - 1) / NT;
+  if (M >= 16 * sm_count)
+    points_analysis_kernel<NT, 4><<<(unsigned)((M + 3) / 4 * passes), kPtThreads, 0, st>>>(M, K, N, B, W, C);
+  else
+    points_analysis_kernel<NT, 1><<<(unsigned)(M * passes), kPtThreads, 0, st>>>(M, K, N, B, W, C);
+}
+
+inline int pass_columns(int N) {
+  const int passes = (N + kPtCols - 1) / kPtCols;
+  return (N + passes - 1) / passes;
+}
+
+}  // namespace
+
+#define AE_PT_PASS(f, nt, ...)                 \
+  switch (nt) {                                \
+    case 1: f<1>(__VA_ARGS__); break;          \
+    case 2: f<2>(__VA_ARGS__); break;          \
+    case 3: f<3>(__VA_ARGS__); break;          \
+    case 4: f<4>(__VA_ARGS__); break;          \
+    case 5: f<5>(__VA_ARGS__); break;          \
+    case 6: f<6>(__VA_ARGS__); break;          \
+    case 7: f<7>(__VA_ARGS__); break;          \
+    default: f<8>(__VA_ARGS__); break;         \
+  }
+
 int points_gemm_synth(const aeolus_plan_impl* p, const double* V, double* out, int ncols, cudaStream_t st) {
-  const long M = p->npoints, K = p->ncol;
-  dim3 grid((unsigned)((M + 63) / 64), (unsigned)((ncols + 31) / 32));
-  dgemm_kernel<true><<<grid, 128, 0, st>>>(M, ncols, K, p->basis, M, V, K, out, M);
-  AE_LAUNCH("dgemm_kernel(synthesis)");
+  ProfScope prof("points_synth_f64", st);
+  AE_PT_PASS(synth_pass, pass_columns(ncols), p->npoints, p->ncol, ncols, p->basis, V, out, st)
+  AE_LAUNCH("points_synth_kernel");
   return AEOLUS_OK;
 }
 
 int points_gemm_analysis(const aeolus_plan_impl* p, const double* W, double* C, int ncols, cudaStream_t st) {
-  const long M = p->ncol, K = p->npoints;
-  dim3 grid((unsigned)((M + 63) / 64), (unsigned)((ncols + 31) / 32));
-  dgemm_kernel<false><<<grid, 128, 0, st>>>(M, ncols, K, p->basis, K, W, K, C, M);
-  AE_LAUNCH("dgemm_kernel(analysis)");
+  ProfScope prof("points_analysis_f64", st);
+  AE_PT_PASS(analysis_pass, pass_columns(ncols), p->ncol, p->npoints, ncols, p->basis, W, C, p->sm_count, st)
+  AE_LAUNCH("points_analysis_kernel");
   return AEOLUS_OK;
 }
 

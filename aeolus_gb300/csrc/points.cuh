@@ -18,19 +18,18 @@ __host__ __device__ inline long col_base(int m, int L) { return m == 0 ? 0 : 2 *
 __host__ __device__ inline long col_cos(int l, int m, int L) { return col_base(m, L) + (l - m); }
 __host__ __device__ inline long col_sin(int l, int m, int L) { return col_base(m, L) + (L + 1 - m) + (l - m); }
 
-// V[(b*NF + f) * ncol + col] from Derive columns (one thread per (b, l, m)).
+// V[(b*NF + f) * ncol + col] from Derive columns (one thread per (b, l, m) of
+// the dense square, orders fastest: coalesced reads, no search for the order).
 template <class Derive>
 __global__ void derive_cols_kernel(int L, int batch, long ncol, double* __restrict__ V, Derive d) {
   constexpr int NF = Derive::NF;
-  const long nlm = (long)(L + 1) * (L + 2) / 2;
+  const long n2 = (long)(L + 1) * (L + 1);
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nlm * batch) return;
-  const int b = (int)(idx / nlm);
-  long r = idx - (long)b * nlm;
-  // r enumerates the m-major triangle: find m with tri_off(m) <= r < tri_off(m+1)
-  int m = 0;
-  while (tri_off(m + 1, L) <= r) ++m;
-  const int l = m + (int)(r - tri_off(m, L));
+  if (idx >= n2 * batch) return;
+  const int b = (int)(idx / n2);
+  const int r = (int)(idx - (long)b * n2);
+  const int l = r / (L + 1), m = r - l * (L + 1);
+  if (m > l) return;
   double2 v[NF];
   d.column(b, l, m, v);
 #pragma unroll
@@ -91,55 +90,123 @@ __global__ void epilogue_cols_kernel(int L, int batch, long ncol, const double* 
   e.finish(b, l, m, acc);
 }
 
-// FP64 tiled GEMM: C[j * ldc + i] = sum_k A(i, k) * B[j * ldb + k], with
-// A(i, k) = A[k * lda + i] (A_COLMAJOR) or A[i * lda + k].
-template <bool A_COLMAJOR>
-__global__ void __launch_bounds__(128) dgemm_kernel(long M, long N, long K, const double* __restrict__ A, long lda,
-                                                   const double* __restrict__ B, long ldb,
-                                                   double* __restrict__ C, long ldc) {
-  constexpr int BM = 64, BN = 32, BK = 16;
-  __shared__ double sA[BK][BM + 1];
-  __shared__ double sB[BK][BN + 1];
-  const long i0 = (long)blockIdx.x * BM, j0 = (long)blockIdx.y * BN;
-  const int tid = threadIdx.x;
-  const int ti = tid % 16, tj = tid / 16;  // 16 x 8 threads, 4 x 4 outputs each
-  double acc[4][4] = {};
-  for (long k0 = 0; k0 < K; k0 += BK) {
-    for (int e = tid; e < BM * BK; e += 128) {
-      int ii, kk;
-      if (A_COLMAJOR) { ii = e % BM; kk = e / BM; } else { kk = e % BK; ii = e / BK; }
-      const long gi = i0 + ii, gk = k0 + kk;
-      double v = 0.0;
-      if (gi < M && gk < K) v = A_COLMAJOR ? A[gk * lda + gi] : A[gi * lda + gk];
-      sA[kk][ii] = v;
-    }
-    for (int e = tid; e < BN * BK; e += 128) {
-      const int kk = e % BK, jj = e / BK;
-      const long gj = j0 + jj, gk = k0 + kk;
-      sB[kk][jj] = (gj < N && gk < K) ? B[gj * ldb + gk] : 0.0;
+// FP64 basis products.  GB300's FP64 pipe does 2 DFMA per clock and SM
+// (629 G/s at 2070 MHz) while HBM delivers 840 G basis values/s, so from two
+// data columns on the products are bound by the multiply-adds themselves:
+// what counts is to issue only useful ones, on every SM.  Each CTA takes
+// exactly the columns there are (NT <= 8 per pass, a template argument) and
+// the contraction is split over its threads, so one field on a small point
+// set (a resolution-4 run: 10,242 product points x 441 columns, 4 + 1 columns
+// per stage) still covers the chip.  The order of each output's sum depends
+// on the plan's sizes only, not on the batch.  Against the square 64 x 32
+// tile this replaces (padded to 32 columns, 7 CTAs in the analysis), a BVE
+// RK4 step of that run went from 29.84 to 0.275 ms; its multiply-adds alone
+// take 0.145 ms at the FP64 rate.
+constexpr int kPtThreads = 256;
+constexpr int kPtCols = 8;      // data columns per pass
+constexpr int kPtRows = 16;     // synthesis: points per CTA (one 128-byte line per basis column)
+constexpr int kPtSlices = kPtThreads / kPtRows;
+constexpr int kPtChunk = 256;   // synthesis: basis columns per staged chunk
+
+// out[n * M + p] = sum_k B[k * M + p] V[n * K + k]: 16 points x 16 slices of
+// the basis columns per CTA; the chunk's coefficients sit in shared memory.
+template <int NT>
+__global__ void __launch_bounds__(kPtThreads) points_synth_kernel(long M, int K, int N, const double* __restrict__ B,
+                                                                  const double* __restrict__ V,
+                                                                  double* __restrict__ out) {
+  __shared__ double sV[kPtChunk][NT];
+  __shared__ double sR[kPtThreads / 32][kPtRows][NT];
+  const unsigned rb = (unsigned)((M + kPtRows - 1) / kPtRows);  // row blocks; passes are the slow grid index
+  const int n0 = (int)(blockIdx.x / rb) * NT, nn = min(NT, N - n0);
+  const long p0 = (long)(blockIdx.x % rb) * kPtRows;
+  const int pt = threadIdx.x % kPtRows, sl = threadIdx.x / kPtRows;
+  const long p = p0 + pt;
+  const double* Bp = B + min(p, M - 1);
+  double acc[NT];
+#pragma unroll
+  for (int q = 0; q < NT; ++q) acc[q] = 0.0;
+  for (int k0 = 0; k0 < K; k0 += kPtChunk) {
+    const int kn = min(kPtChunk, K - k0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < NT * kPtChunk; e += kPtThreads) {
+      const int k = e % kPtChunk, q = e / kPtChunk;
+      if (k < kn) sV[k][q] = q < nn ? V[(long)(n0 + q) * K + k0 + k] : 0.0;
     }
     __syncthreads();
+#pragma unroll 8
+    for (int k = sl; k < kn; k += kPtSlices) {
+      const double bv = __ldg(Bp + (long)(k0 + k) * M);
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      double a[4], bv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = sA[kk][ti + 16 * u];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) bv[v] = sB[kk][tj + 8 * v];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], bv[v], acc[u][v]);
+      for (int q = 0; q < NT; ++q) acc[q] = fma(bv, sV[k][q], acc[q]);
     }
-    __syncthreads();
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int q = 0; q < NT; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], kPtRows);
+  if ((threadIdx.x & 31) < kPtRows)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const long gi = i0 + ti + 16 * u, gj = j0 + tj + 8 * v;
-      if (gi < M && gj < N) C[gj * ldc + gi] = acc[u][v];
+    for (int q = 0; q < NT; ++q) sR[threadIdx.x >> 5][pt][q] = acc[q];
+  __syncthreads();
+  for (int e = threadIdx.x; e < kPtRows * NT; e += kPtThreads) {
+    const int r = e % kPtRows, q = e / kPtRows;
+    const long pr = p0 + r;
+    if (q >= nn || pr >= M) continue;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < kPtThreads / 32; ++w) v += sR[w][r][q];
+    out[(long)(n0 + q) * M + pr] = v;
+  }
+}
+
+// C[n * M + c] = sum_p B[c * K + p] W[n * K + p]: CT basis columns per CTA,
+// its threads stride over the points (contiguous in B and W).
+template <int NT, int CT>
+__global__ void __launch_bounds__(kPtThreads) points_analysis_kernel(int M, long K, int N, const double* __restrict__ B,
+                                                                     const double* __restrict__ W,
+                                                                     double* __restrict__ C) {
+  __shared__ double sR[kPtThreads / 32][CT * NT];
+  const unsigned cb = (unsigned)((M + CT - 1) / CT);
+  const int n0 = (int)(blockIdx.x / cb) * NT, nn = min(NT, N - n0);
+  const int c0 = (int)(blockIdx.x % cb) * CT;
+  const double* Bc[CT];
+  const double* Wn[NT];
+#pragma unroll
+  for (int i = 0; i < CT; ++i) Bc[i] = B + (long)min(c0 + i, M - 1) * K;
+#pragma unroll
+  for (int q = 0; q < NT; ++q) Wn[q] = W + (long)(n0 + min(q, nn - 1)) * K;
+  double acc[CT][NT];
+#pragma unroll
+  for (int i = 0; i < CT; ++i)
+#pragma unroll
+    for (int q = 0; q < NT; ++q) acc[i][q] = 0.0;
+#pragma unroll 2
+  for (long p = threadIdx.x; p < K; p += kPtThreads) {
+    double b[CT], w[NT];
+#pragma unroll
+    for (int i = 0; i < CT; ++i) b[i] = __ldg(Bc[i] + p);
+#pragma unroll
+    for (int q = 0; q < NT; ++q) w[q] = __ldg(Wn[q] + p);
+#pragma unroll
+    for (int i = 0; i < CT; ++i)
+#pragma unroll
+      for (int q = 0; q < NT; ++q) acc[i][q] = fma(b[i], w[q], acc[i][q]);
+  }
+#pragma unroll
+  for (int i = 0; i < CT; ++i)
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+      double v = acc[i][q];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) == 0) sR[threadIdx.x >> 5][i * NT + q] = v;
     }
+  __syncthreads();
+  for (int e = threadIdx.x; e < CT * NT; e += kPtThreads) {
+    const int i = e / NT, q = e % NT;
+    if (q >= nn || c0 + i >= M) continue;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < kPtThreads / 32; ++w) v += sR[w][e];
+    C[(long)(n0 + q) * M + c0 + i] = v;
+  }
 }
 
 int points_gemm_synth(const aeolus_plan_impl* p, const double* V, double* out, int ncols, cudaStream_t st);
