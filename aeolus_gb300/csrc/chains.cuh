@@ -90,6 +90,7 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
     ra.G = G;
     ra.gblk = Pw::NOUT;
     ra.status = status;
+    ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
     if ((s = launch_rows<Pw, kInF, kOutG>(p, pw, ra, st))) return s;
     return launch_split_anal(p, e, G, Pw::NOUT, batch, scratch, st);
   } else if (p->kind == kGauss) {
@@ -112,6 +113,7 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
     ra.G = G;
     ra.gblk = Pw::NOUT;
     ra.status = status;
+    ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
     if ((s = launch_rows<Pw, kInF, kOutG>(p, pw, ra, st))) return s;
     return split ? launch_split_anal(p, e, G, Pw::NOUT, batch, scratch, st)
                  : launch_analysis(p, e, FG, NB, batch, st);

@@ -354,6 +354,11 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     ra.batch = E->batch[k];
     ra.FG = reinterpret_cast<double2*>(chain[k]);
     ra.nblk = NB;
+    ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
+    if (E->split) {  // compact G blocks after F, as in run_full_chain
+      ra.G = reinterpret_cast<double2*>(chain[k] + align256(fg_bytes(p, NB, E->batch[k])));
+      ra.gblk = NOUT;
+    }
     row_args(p, ra);
     if (E->split) ra.fft = p->fftx;
     const int kind = E->split ? split_row_kind(p) : kRowsRuntime;
@@ -421,12 +426,14 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     const aeolus_plan_impl* p = E->plan[k];
     const int B = E->batch[k];
     double2* FG = reinterpret_cast<double2*>(chain[k]);
-    void* scratch = chain[k] + align256(fg_bytes(p, NB, B));
+    char* G = chain[k] + align256(fg_bytes(p, NB, B));
+    void* scratch = G + align256(fg_bytes(p, NOUT, B));
     const SplitParts r1 = split_synth_parts<NS>(p, B, scratch);
-    const SplitParts r2 = split_anal_parts<NOUT>(p, B, scratch);
+    const int top = EpiTop<Epi>::top(p->lmax);
+    const SplitParts r2 = split_anal_parts<NOUT>(p, B, scratch, top);
     const SDerive sd = M::split_derive(der[k]);
     grouped_add(gss, SliceSynthArg<SDerive>{r1.dm, p->split->kcum, B, r1.mb, sd, r1.digits, r1.ecol}, r1.grid);
-    grouped_add(gsa, SliceAnalArg{r2.dm, B, r2.mb, NB, reinterpret_cast<const long long*>(FG), r2.digits, r2.ecol},
+    grouped_add(gsa, SliceAnalArg{r2.dm, B, r2.mb, NOUT, reinterpret_cast<const long long*>(G), r2.digits, r2.ecol},
                 r2.grid);
     sm_ss = std::max(sm_ss, r1.smem);
     sm_sa = std::max(sm_sa, r2.smem);
@@ -436,7 +443,7 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     esyn.e[k] = SEpi{r1.dm, p->split->esyn, r1.ecol, NB, reinterpret_cast<float4*>(FG)};
     esyn.e[k].ir_hi = (float)SynthOut<SDerive>::ir(sd);
     esyn.e[k].ir_lo = (float)(SynthOut<SDerive>::ir(sd) - (double)esyn.e[k].ir_hi);
-    const AnalSched sa{r2.dm, p->split->pana, r2.digits};
+    const AnalSched sa{r2.dm, p->split->pana, r2.digits, top};
     tana.s[k] = sa;
     tana.start[k + 1] = tana.start[k] + sa.count_host();
     eana.e[k] = AnalEpi<Epi>{r2.dm, p->split->eana, r2.ecol, B, epi[k]};

@@ -13,9 +13,27 @@
 //             consumes a_lm for l >= m; zero(b, l, m) handles l < m slots.
 #pragma once
 
+#include <type_traits>
+#include <utility>
+
 #include "common.cuh"
 
 namespace aeolus {
+
+// Highest degree and order an epilogue uses of the analysed fields.  The
+// tendencies and the Jacobian cut their products to the 2/3 rule (degrees and
+// orders up to 2L/3), so 56 % of the triangle of an analysis would be thrown
+// away: their epilogues declare kCut, the row stage then writes no order above
+// the cut and the contraction runs over the kept triangle only (an epilogue
+// still visits every slot, with zeros for the cut ones).
+template <class E, class = void>
+struct EpiTop {
+  __host__ __device__ static int top(int L) { return L; }
+};
+template <class E>
+struct EpiTop<E, std::enable_if_t<E::kCut>> {
+  __host__ __device__ static int top(int L) { return (2 * L) / 3; }
+};
 
 struct LegArgs {
   int L, nlat, nh, batch, bc;

@@ -33,6 +33,7 @@ struct JacDerive {  // a_lam, a_snt, b_lam, b_snt
 
 struct TruncEpi {  // 2/3-truncated store
   static constexpr int NF = 1;
+  static constexpr bool kCut = true;
   double2* out;
   int L;
   __device__ void finish(int b, int l, int m, const double2* acc) const {

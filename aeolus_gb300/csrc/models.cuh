@@ -205,6 +205,7 @@ struct Rk4 {
 
 struct BveEpi {  // -trunc(A J) + nu lap zeta (+ forcing), l = 0 row zero
   static constexpr int NF = 1;
+  static constexpr bool kCut = true;
   Spec s;
   const double2* zeta;     // stage input
   const double2* forcing;  // optional
@@ -498,6 +499,7 @@ struct SweDerive7 {
 // through the split contraction shrink ~10x (|zeta| << |f|).
 struct SweEpi {
   static constexpr int NF = 4;
+  static constexpr bool kCut = true;
   Spec s;
   const double2* state;  // stage input [b][3][L+1][L+1]
   double phi0, nu4;

@@ -36,6 +36,7 @@ struct RowArgs {
   double* gout;
   long gout_b, gout_f;
   unsigned* status;       // optional per-member state bits
+  int drop;               // kOutG: orders above L - drop are not written (EpiTop)
 };
 
 // x / d through the stage's 32-bit reciprocal (exact for x * d < 2^32).
@@ -242,7 +243,7 @@ __device__ __forceinline__ void row_body(const RowArgs& a, const Pw& pw, int bx,
       double2* zother = (zin == buf0) ? buf1 : buf0;
       double2* Z = fft_run<false>(zin, zother, NOUT, ns, a.fft, a.tw);
       // R_q = (Z_q + conj Z_{n-q})/2 - (i/2) e^{-2 pi i q/N} (Z_q - conj Z_{n-q})
-      for (int idx = threadIdx.x; idx < NOUT * ldm; idx += blockDim.x) {
+      for (int idx = threadIdx.x; idx < NOUT * (ldm - a.drop); idx += blockDim.x) {
         const int q = idx / NOUT, f = idx - q * NOUT;  // fields fastest: contiguous global writes
         const double2* Zf = Z + (long)f * ns;
         double2 zq = Zf[q];
@@ -254,7 +255,7 @@ __device__ __forceinline__ void row_body(const RowArgs& a, const Pw& pw, int bx,
         block[(long)q * sq + f] = cscale(wj, R);
       }
     } else {
-      for (int idx = threadIdx.x; idx < NOUT * ldm; idx += blockDim.x) {
+      for (int idx = threadIdx.x; idx < NOUT * (ldm - a.drop); idx += blockDim.x) {
         const int q = idx / NOUT, f = idx - q * NOUT;
         const double* x = xout + (long)f * 2 * ns;
         double sr = 0.0, si = 0.0;

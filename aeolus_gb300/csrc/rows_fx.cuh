@@ -480,7 +480,7 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
     __syncthreads();
     // rows to fixed point inside the first stage; output in digit-reversed order
     FFT::template run<false>(zout, NOUT, ns, a.fft, twfx, kc, s_pa, s_pb);
-    for (int idx = threadIdx.x; idx < NOUT * ldm; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < NOUT * (ldm - a.drop); idx += blockDim.x) {
       const int q = idx / NOUT, f = idx - q * NOUT;  // fields fastest: contiguous global writes
       const cfx* Zf = zout + (long)f * ns;
       const cfx zq = Zf[__ldg(&a.irev[q])];
@@ -493,7 +493,7 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
       reinterpret_cast<longlong2*>(oblock)[(long)q * sqo + f] = make_longlong2(pk_pack(R2.re, e), pk_pack(R2.im, e));
     }
   } else {
-    for (int idx = threadIdx.x; idx < NOUT * ldm; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < NOUT * (ldm - a.drop); idx += blockDim.x) {
       const int q = idx / NOUT, f = idx - q * NOUT;
       const df* x = xout + (long)f * 2 * ns;
       df sr = df{0.f, 0.f}, si = df{0.f, 0.f};
@@ -777,7 +777,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
       const int f = tid % NOUT;
       const int e = s_in[f] - 1;  // R2 / 2 in units of 2^S
       const cfx* Zf = buf0 + f * fs;
-      for (int q = tid / NOUT; q < ldm; q += QSO) {
+      for (int q = tid / NOUT; q < ldm - a.drop; q += QSO) {
         const cfx zq = Zf[Row::swz(Row::rev(q))];
         const cfx zn = fx_conj(Zf[Row::swz(Row::rev(q == 0 ? 0 : n - q))]);
         const cfx E2 = fx_add(zq, zn);

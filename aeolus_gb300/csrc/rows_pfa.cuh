@@ -514,7 +514,7 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
 #pragma unroll 1
         for (int p = 0; p < 2 * R0; ++p) {
           const int q = (p < R0 ? c : g1) + (p < R0 ? p : p - R0) * P;
-          if (q <= L) pfa_post<S>(Z, q, e, twfx, ob + (long)q * sqo, s_spec);
+          if (q <= L - a.drop) pfa_post<S>(Z, q, e, twfx, ob + (long)q * sqo, s_spec);
         }
       }
     }

@@ -859,13 +859,14 @@ struct AnalSched {
   SplitDims dm;
   const __nv_bfloat16* pana;
   const __nv_bfloat16* dana;
+  int top;  // orders above it are not contracted (EpiTop): their tiles only run the epilogue, with zeros
   __host__ __device__ int count() const { return ana_row_tiles(dm.L) * dm.ntiles; }
   int count_host() const { return count(); }
   __device__ TcTile tile(int t) const {
     const int rt = t / dm.ntiles, nt = t - rt * dm.ntiles;
     int m, mt;
     ana_row_tile(dm.L, rt, m, mt);
-    return TcTile{pana + pana_tile(dm.NK, rt), dana + dana_tile(dm, m, nt), dm.NK / kKC};
+    return TcTile{pana + pana_tile(dm.NK, rt), dana + dana_tile(dm, m, nt), m <= top ? dm.NK / kKC : 0};
   }
 };
 
@@ -1002,7 +1003,7 @@ SplitParts split_synth_parts(const aeolus_plan_impl* p, int batch, void* scratch
 }
 
 template <int NF>
-SplitParts split_anal_parts(const aeolus_plan_impl* p, int batch, void* scratch) {
+SplitParts split_anal_parts(const aeolus_plan_impl* p, int batch, void* scratch, int top) {
   SplitParts r;
   r.dm = split_dims(p, batch * NF * 2);
   char* w = static_cast<char*>(scratch);
@@ -1011,7 +1012,7 @@ SplitParts split_anal_parts(const aeolus_plan_impl* p, int batch, void* scratch)
   r.ecol = reinterpret_cast<int*>(w);
   r.mb = slice_members(NF, r.dm.nlat + 1, p->tune_slice_mb_anal);
   r.smem = (size_t)r.mb * NF * 2 * (r.dm.nlat | 1) * 8;
-  r.grid = dim3(r.dm.L + 1, (batch + r.mb - 1) / r.mb);
+  r.grid = dim3(top + 1, (batch + r.mb - 1) / r.mb);
   return r;
 }
 
@@ -1047,7 +1048,8 @@ template <class Epi>
 int launch_split_anal(const aeolus_plan_impl* p, const Epi& e, const double2* FG, int nblk, int batch, void* scratch,
                       cudaStream_t st) {
   constexpr int NF = Epi::NF;
-  const SplitParts r = split_anal_parts<NF>(p, batch, scratch);
+  const int top = EpiTop<Epi>::top(p->lmax);
+  const SplitParts r = split_anal_parts<NF>(p, batch, scratch, top);
   auto k1 = split_anal_slice_kernel<NF>;
   int s = allow_smem(k1, r.smem);
   if (s) return s;
@@ -1060,7 +1062,7 @@ int launch_split_anal(const aeolus_plan_impl* p, const Epi& e, const double2* FG
   const size_t sm2 = tc_smem_bytes();
   auto k2 = tc_persistent_kernel<AnalSched, AnalEpi<Epi>>;
   if ((s = allow_smem(k2, sm2))) return s;
-  const AnalSched sc{r.dm, p->split->pana, r.digits};
+  const AnalSched sc{r.dm, p->split->pana, r.digits, top};
   const AnalEpi<Epi> ep{r.dm, p->split->eana, r.ecol, batch, e};
   ProfScope prof("tc_anal_bf16x6", st);
   launch_pdl(k2, dim3(tc_grid(p, sc.count_host())), dim3(tc_threads<AnalEpi<Epi>>()), sm2, st, sc, ep, p->split->err);
