@@ -92,11 +92,11 @@ struct SliceAnalArg {
   int* ecol;
 };
 
-template <class Derive, int CPT>
+template <class Derive>
 __global__ void __launch_bounds__(256) g_legendre_synth(Grouped<SynthArg<Derive>> g) {
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
-  legendre_synth_body<Derive, CPT>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
+  legendre_synth_body<Derive>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
 }
 
 template <class Epi>
@@ -380,17 +380,17 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
       double2* FG = reinterpret_cast<double2*>(chain[k]);
       const LegCfg cs = synth_cfg<Derive>(p, E->batch[k]);
       const LegCfg ca = analysis_cfg<Epi>(p, E->batch[k]);
-      grouped_add(gs, SynthArg<Derive>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], cs.bc, p->P, p->PT, FG, NB},
+      grouped_add(gs, SynthArg<Derive>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], cs.bc, cs.ss, p->P, p->PT, FG, NB},
                                        der[k]},
                   cs.grid);
-      grouped_add(ga, AnalArg<Epi>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], ca.bc, p->P, p->PT, FG, NB}, epi[k]},
+      grouped_add(ga, AnalArg<Epi>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], ca.bc, ca.ss, p->P, p->PT, FG, NB}, epi[k]},
                   ca.grid);
       sm_s = std::max(sm_s, cs.smem);
       sm_a = std::max(sm_a, ca.smem);
       thr_s = std::max(thr_s, cs.threads);
       thr_a = std::max(thr_a, ca.threads);
     }
-    auto k1 = g_legendre_synth<Derive, kSynthCPT>;
+    auto k1 = g_legendre_synth<Derive>;
     auto k2 = g_rows<Pw>;
     auto k3 = g_legendre_analysis<Epi>;
     if ((s = allow_smem(k1, sm_s)) || (s = allow_smem(k2, sm_rows)) || (s = allow_smem(k3, sm_a))) return s;

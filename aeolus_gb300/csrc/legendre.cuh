@@ -37,32 +37,45 @@ struct EpiTop<E, std::enable_if_t<E::kCut>> {
 
 struct LegArgs {
   int L, nlat, nh, batch, bc;
+  int ss;            // CTAs that share the items of one (order pair, member chunk)
   const double* P;   // synthesis table (row index fastest)
   const double* PT;  // analysis table (degree fastest)
   double2* FG;       // F / G blocks [b][j][nblk][L+1]
   int nblk;
 };
 
-inline int n_pairs(int L) { return L / 2 + 1; }
+__host__ __device__ inline int n_pairs(int L) { return L / 2 + 1; }
 
-template <class Derive, int CPT>
+// Both kernels are bound by the FP64 pipe (2 DFMA per clock and SM: a warp's
+// DFMA occupies its sub-partition for 64 cycles, so one warp with two
+// independent sums per sub-partition already saturates it and the loads that
+// feed it are free).  What costs is idle lanes and idle SMs, so the work items
+// are the smallest independent ones, packed densely over the threads:
+//   synthesis  (northern row, data column) per item;
+//   analysis   (degree, one of JS row slices) per item, the slices added
+//              through shared memory; JS depends on the grid alone, so a
+//              member's result does not depend on the batch;
+// and the items of one (order pair, member chunk) are shared by `ss` CTAs when
+// there are too few of those to fill the chip (leg_shares, pipeline.cuh).
+// FP64 SWE RK4 steps with these kernels and the kept-triangle analysis: one
+// member at 128 x 256, l_max 85 505 -> 377 us (analysis 30.4 -> 14.6 us per
+// stage), 8 members at 192 x 384, l_max 127 3.30 -> 2.91 ms (142 -> 93 us).
+template <class Derive>
 __device__ __forceinline__ void legendre_synth_body(const LegArgs& a, const Derive& d, int bx, int by) {
   constexpr int NF = Derive::NF;
   extern __shared__ double2 s_a[];
-  const int L = a.L, nh = a.nh, ldm = L + 1;
-  const int i = bx;
+  const int L = a.L, nh = a.nh;
+  const int i = bx / a.ss;
   const int mA = i, mB = L - i;
   const bool two = mB != mA;
   const int KA = L + 1 - mA, KB = two ? L + 1 - mB : 0;
-  const int b0 = by * a.bc;
+  const int share = bx % a.ss, b0 = by * a.bc;
   const int nb = min(a.bc, a.batch - b0);
   const int ncols = nb * NF;
-  const int ngroups = (ncols + CPT - 1) / CPT;
-  const int ncp = ngroups * CPT;  // padded column count
-  double2* sA = s_a;                 // [ncp][KA]
-  double2* sB = s_a + (long)ncp * KA;  // [ncp][KB]
+  double2* sA = s_a;                   // [ncols][KA]
+  double2* sB = s_a + (long)ncols * KA;  // [ncols][KB]
 
-  // derived coefficient columns of both orders (zero padding columns)
+  // derived coefficient columns of both orders
   for (int idx = threadIdx.x; idx < nb * (KA + KB); idx += blockDim.x) {
     const int bl = idx / (KA + KB);
     const int t = idx - bl * (KA + KB);
@@ -76,91 +89,78 @@ __device__ __forceinline__ void legendre_synth_body(const LegArgs& a, const Deri
 #pragma unroll
     for (int f = 0; f < NF; ++f) dst[(long)(bl * NF + f) * K + tt] = v[f];
   }
-  for (int idx = threadIdx.x; idx < (ncp - ncols) * (KA + KB); idx += blockDim.x) {
-    const int c = ncols + idx / (KA + KB);
-    const int t = idx % (KA + KB);
-    if (t < KA) sA[(long)c * KA + t] = make_double2(0.0, 0.0);
-    else sB[(long)c * KB + (t - KA)] = make_double2(0.0, 0.0);
-  }
   __syncthreads();
 
-  for (int item = threadIdx.x; item < nh * ngroups; item += blockDim.x) {
-    const int jn = item % nh, g = item / nh;
-    const int c0 = g * CPT;
+  const int items = nh * ncols, per = (items + a.ss - 1) / a.ss;
+  for (int item = share * per + threadIdx.x; item < min(items, (share + 1) * per); item += blockDim.x) {
+    const int c = item / nh, jn = item - c * nh;
     const int jS = a.nlat - 1 - jn;
+    const int bl = c / NF, f = c - bl * NF;
     for (int pass = 0; pass < (two ? 2 : 1); ++pass) {
       const int m = pass ? mB : mA;
       const int K = pass ? KB : KA;
-      const double2* sc = (pass ? sB : sA) + (long)c0 * K;
+      const double2* sc = (pass ? sB : sA) + (long)c * K;
       const double* Pm = a.P + tri_off(m, L) * nh + jn;
-      double2 E[CPT], O[CPT];
-#pragma unroll
-      for (int q = 0; q < CPT; ++q) E[q] = O[q] = make_double2(0.0, 0.0);
+      double2 E = make_double2(0.0, 0.0), O = E;
       int t = 0;
+#pragma unroll 4
       for (; t + 1 < K; t += 2) {
         const double pe = __ldg(Pm + (long)t * nh);
         const double po = __ldg(Pm + (long)(t + 1) * nh);
-#pragma unroll
-        for (int q = 0; q < CPT; ++q) {
-          const double2 ae = sc[(long)q * K + t];
-          const double2 ao = sc[(long)q * K + t + 1];
-          E[q].x = fma(pe, ae.x, E[q].x);
-          E[q].y = fma(pe, ae.y, E[q].y);
-          O[q].x = fma(po, ao.x, O[q].x);
-          O[q].y = fma(po, ao.y, O[q].y);
-        }
+        const double2 ae = sc[t], ao = sc[t + 1];
+        E.x = fma(pe, ae.x, E.x);
+        E.y = fma(pe, ae.y, E.y);
+        O.x = fma(po, ao.x, O.x);
+        O.y = fma(po, ao.y, O.y);
       }
       if (t < K) {
         const double pe = __ldg(Pm + (long)t * nh);
-#pragma unroll
-        for (int q = 0; q < CPT; ++q) {
-          const double2 ae = sc[(long)q * K + t];
-          E[q].x = fma(pe, ae.x, E[q].x);
-          E[q].y = fma(pe, ae.y, E[q].y);
-        }
+        const double2 ae = sc[t];
+        E.x = fma(pe, ae.x, E.x);
+        E.y = fma(pe, ae.y, E.y);
       }
-#pragma unroll
-      for (int q = 0; q < CPT; ++q) {
-        const int c = c0 + q;
-        if (c >= ncols) break;
-        const int bl = c / NF, f = c - bl * NF;
-        const long bb = b0 + bl;
-        a.FG[fg_index(bb, m, f, jn, L, a.nblk, a.nlat)] = cadd(E[q], O[q]);
-        if (jS != jn) a.FG[fg_index(bb, m, f, jS, L, a.nblk, a.nlat)] = csub(E[q], O[q]);
-      }
+      const long bb = b0 + bl;
+      a.FG[fg_index(bb, m, f, jn, L, a.nblk, a.nlat)] = cadd(E, O);
+      if (jS != jn) a.FG[fg_index(bb, m, f, jS, L, a.nblk, a.nlat)] = csub(E, O);
     }
   }
 }
 
-template <class Derive, int CPT>
+template <class Derive>
 __global__ void __launch_bounds__(256) legendre_synth_kernel(LegArgs a, Derive d) {
-  legendre_synth_body<Derive, CPT>(a, d, blockIdx.x, blockIdx.y);
+  legendre_synth_body<Derive>(a, d, blockIdx.x, blockIdx.y);
 }
 
-template <class Derive, int CPT>
+template <class Derive>
 inline size_t synth_smem_bytes(int L, int bc) {
-  const int ncols = bc * Derive::NF;
-  const int ncp = (ncols + CPT - 1) / CPT * CPT;
-  return (size_t)ncp * (L + 2) * sizeof(double2);
+  return (size_t)bc * Derive::NF * (L + 2) * sizeof(double2);
+}
+
+// Row slices per degree of the analysis (a power of two, from the grid and the
+// field count alone).  Rows that fill most of the shared memory by themselves
+// (above 160 KB) leave no room for partial sums: one slice, finished directly.
+__host__ __device__ inline int leg_row_slices(int nh, int nf) {
+  return (long)64 * nf * nh > 160 * 1024 ? 1 : nh >= 32 ? 8 : nh >= 8 ? 4 : 1;
 }
 
 template <class Epi>
 __device__ __forceinline__ void legendre_analysis_body(const LegArgs& a, const Epi& e, int bx, int by) {
   constexpr int NF = Epi::NF;
-  extern __shared__ double2 s_g[];  // [2 orders][nb][NF][2 parities][nh]
-  const int L = a.L, nh = a.nh, ldm = L + 1;
-  const int i = bx;
-  const int mA = i, mB = L - i;
+  extern __shared__ double2 s_g[];  // [2 orders][nb][NF][2 parities][nh], then [items / JS][JS][NF] partial sums
+  const int L = a.L, nh = a.nh, top = EpiTop<Epi>::top(L);
+  const int i = bx / a.ss;
+  const int mA = i, mB = top - i;
   const bool two = mB != mA;
-  const int KA = L + 1 - mA, KB = two ? L + 1 - mB : 0;
-  const int b0 = by * a.bc;
+  const int KA = top + 1 - mA, KB = two ? top + 1 - mB : 0;
+  const int share = bx % a.ss, b0 = by * a.bc;
   const int nb = min(a.bc, a.batch - b0);
+  const int JS = leg_row_slices(nh, NF);
   const long per_order = (long)a.bc * NF * 2 * nh;
 
   for (int idx = threadIdx.x; idx < (two ? 2 : 1) * nb * NF * nh; idx += blockDim.x) {
     int r = idx;
-    const int jn = r % nh; r /= nh;
     const int f = r % NF; r /= NF;
+    const int jn = r % nh; r /= nh;
     const int bl = r % nb; r /= nb;
     const int which = r;
     const int m = which ? mB : mA;
@@ -174,21 +174,27 @@ __device__ __forceinline__ void legendre_analysis_body(const LegArgs& a, const E
   }
   __syncthreads();
 
+  // degrees of this CTA: [d0, d1) of the nb (KA + KB) (member, degree) pairs
   const int KT = KA + KB;
-  for (int item = threadIdx.x; item < nb * KT; item += blockDim.x) {
-    const int bl = item / KT;
-    const int t0 = item - bl * KT;
+  const int per = (nb * KT + a.ss - 1) / a.ss;
+  const int d0 = share * per, d1 = min(nb * KT, d0 + per);
+  double2* part = s_g + 2 * per_order;
+  for (int item = threadIdx.x; item < (d1 - d0) * JS; item += blockDim.x) {
+    const int di = item / JS, js = item - di * JS;
+    const int bl = (d0 + di) / KT;
+    const int t0 = d0 + di - bl * KT;
     const bool isA = t0 < KA;
     const int m = isA ? mA : mB;
     const int t = isA ? t0 : t0 - KA;
-    const int K = isA ? KA : KB;
+    const int K = L + 1 - m;
     const int par = t & 1;
     const double2* sg = s_g + (isA ? 0 : per_order) + ((long)bl * NF * 2 + par) * nh;
     const double* pt = a.PT + tri_off(m, L) * nh + t;
     double2 acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = make_double2(0.0, 0.0);
-    for (int jn = 0; jn < nh; ++jn) {
+#pragma unroll 4
+    for (int jn = js; jn < nh; jn += JS) {
       const double p = __ldg(pt + (long)jn * K);
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
@@ -197,15 +203,44 @@ __device__ __forceinline__ void legendre_analysis_body(const LegArgs& a, const E
         acc[f].y = fma(p, g.y, acc[f].y);
       }
     }
-    e.finish(b0 + bl, m + t, m, acc);
+    if (JS == 1) {
+      e.finish(b0 + bl, m + t, m, acc);
+    } else {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) part[(long)item * NF + f] = acc[f];
+    }
   }
-  // slots l < m of the two columns
-  for (int idx = threadIdx.x; idx < nb * (mA + (two ? mB : 0)); idx += blockDim.x) {
-    const int per = mA + (two ? mB : 0);
-    const int bl = idx / per;
-    const int r = idx - bl * per;
-    if (r < mA) e.zero(b0 + bl, r, mA);
-    else e.zero(b0 + bl, r - mA, mB);
+  if (JS > 1) {
+    __syncthreads();
+    // the slices of one (degree, field) added in slice order, dense over the threads
+    for (int idx = threadIdx.x; idx < (d1 - d0) * NF; idx += blockDim.x) {
+      const int di = idx / NF, f = idx - di * NF;
+      double2* q = part + (long)di * JS * NF + f;
+      double2 s = q[0];
+      for (int js = 1; js < JS; ++js) s = cadd(s, q[js * NF]);
+      q[0] = s;
+    }
+    __syncthreads();
+    for (int di = threadIdx.x; di < d1 - d0; di += blockDim.x) {
+      const int bl = (d0 + di) / KT;
+      const int t0 = d0 + di - bl * KT;
+      const bool isA = t0 < KA;
+      const int m = isA ? mA : mB;
+      const double2* q = part + (long)di * JS * NF;
+      double2 acc[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) acc[f] = q[f];
+      e.finish(b0 + bl, m + (isA ? t0 : t0 - KA), m, acc);
+    }
+  }
+  // the slots outside the kept triangle, shared by every CTA of these members
+  const int n2 = (L + 1) * (L + 1), ncta = n_pairs(top) * a.ss;
+  const double2 none[NF] = {};
+  for (int idx = bx * blockDim.x + threadIdx.x; idx < nb * n2; idx += ncta * blockDim.x) {
+    const int bl = idx / n2, r = idx - bl * n2;
+    const int l = r / (L + 1), m = r - l * (L + 1);
+    if (m > l) e.zero(b0 + bl, l, m);
+    else if (l > top) e.finish(b0 + bl, l, m, none);
   }
 }
 
@@ -215,8 +250,11 @@ __global__ void __launch_bounds__(256) legendre_analysis_kernel(LegArgs a, Epi e
 }
 
 template <class Epi>
-inline size_t analysis_smem_bytes(int nh, int bc) {
-  return (size_t)2 * bc * Epi::NF * 2 * nh * sizeof(double2);
+inline size_t analysis_smem_bytes(int L, int nh, int bc, int ss) {
+  const int top = EpiTop<Epi>::top(L);
+  const size_t degrees = ((size_t)bc * (top + 2) + ss - 1) / ss;
+  const int js = leg_row_slices(nh, Epi::NF);
+  return ((size_t)2 * bc * Epi::NF * 2 * nh + (js > 1 ? degrees * js * Epi::NF : 0)) * sizeof(double2);
 }
 
 // ------------------------------------------------------------ plain functors

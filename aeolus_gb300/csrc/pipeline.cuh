@@ -13,8 +13,6 @@
 
 namespace aeolus {
 
-constexpr int kSynthCPT = 3;
-
 inline int pick_bc(int L, int batch) {
   const long ctas = (long)n_pairs(L) * batch;
   int bc = (int)std::max(1L, std::min(4L, ctas / 608));
@@ -42,28 +40,57 @@ inline int round_threads(long items, int lo, int hi) {
 // plan's tune_* fields; 0 keeps the built-in heuristic).
 struct LegCfg {
   int bc;          // members per CTA
+  int ss;          // CTAs per (order pair, member chunk)
   int threads;
   size_t smem;
   dim3 grid;
 };
 
+// Warps of a CTA with `warps` warps of items: at most 8, with the fewest idle
+// ones in the last round.
+inline int leg_warps(int warps) {
+  int best = 1, cost = warps;
+  for (int w = 2; w <= 8; ++w) {
+    const int c = (warps + w - 1) / w * w;
+    if (c <= cost || best < 4) best = w, cost = c;
+  }
+  return best;
+}
+
+// CTAs that share one (order pair, member chunk) of `warps` warps of items:
+// six CTAs per SM even out the last wave (8 members at l_max 127: 512 pairs
+// on 152 SMs are 4 rounds for 3.4 of work); no CTA gets fewer than two warps,
+// and its share of the columns' derivation stays a few percent.
+inline int leg_shares(const aeolus_plan_impl* p, long ctas, int warps) {
+  const long want = (6L * p->sm_count + ctas - 1) / std::max(ctas, 1L);
+  return (int)std::max(1L, std::min<long>(want, warps / 2));
+}
+
 template <class Derive>
 LegCfg synth_cfg(const aeolus_plan_impl* p, int batch) {
   const int L = p->lmax;
   int bc = p->tune_bc_synth > 0 ? std::min(p->tune_bc_synth, std::max(batch, 1)) : pick_bc(L, batch);
-  while (bc > 1 && synth_smem_bytes<Derive, kSynthCPT>(L, bc) > 200 * 1024) --bc;
-  const int ngroups = (bc * Derive::NF + kSynthCPT - 1) / kSynthCPT;
-  return LegCfg{bc, round_threads((long)p->nh * ngroups, 64, 256), synth_smem_bytes<Derive, kSynthCPT>(L, bc),
-                dim3(n_pairs(L), (batch + bc - 1) / bc)};
+  while (bc > 1 && synth_smem_bytes<Derive>(L, bc) > 200 * 1024) --bc;
+  const int gy = (batch + bc - 1) / bc, items = p->nh * bc * Derive::NF;
+  const int ss = leg_shares(p, (long)n_pairs(L) * gy, (items + 31) / 32);
+  const int per = (items + ss - 1) / ss;
+  return LegCfg{bc, ss, 32 * leg_warps((per + 31) / 32), synth_smem_bytes<Derive>(L, bc), dim3(n_pairs(L) * ss, gy)};
 }
 
 template <class Epi>
 LegCfg analysis_cfg(const aeolus_plan_impl* p, int batch) {
-  const int L = p->lmax;
-  int bc = p->tune_bc_anal > 0 ? std::min(p->tune_bc_anal, std::max(batch, 1)) : pick_bc(L, batch);
-  while (bc > 1 && analysis_smem_bytes<Epi>(p->nh, bc) > 220 * 1024) --bc;
-  return LegCfg{bc, round_threads((long)bc * (L + 2), 64, 256), analysis_smem_bytes<Epi>(p->nh, bc),
-                dim3(n_pairs(L), (batch + bc - 1) / bc)};
+  const int L = p->lmax, top = EpiTop<Epi>::top(L), js = leg_row_slices(p->nh, Epi::NF);
+  int bc = p->tune_bc_anal > 0 ? std::min(p->tune_bc_anal, std::max(batch, 1)) : pick_bc(top, batch);
+  while (bc > 1 && analysis_smem_bytes<Epi>(L, p->nh, bc, 1) > 160 * 1024) --bc;
+  const int gy = (batch + bc - 1) / bc, degrees = bc * (top + 2), q = 32 / js;  // q degrees fill a warp
+  const int want = leg_shares(p, (long)n_pairs(top) * gy, (degrees * js + 31) / 32);
+  int per = (degrees + want - 1) / want;
+  per = std::max(std::min(q, degrees), per / q * q);
+  int ss = (degrees + per - 1) / per;
+  while (ss < degrees && analysis_smem_bytes<Epi>(L, p->nh, bc, ss) > 220 * 1024) ++ss;  // partial sums that fit
+  per = (degrees + ss - 1) / ss;
+  return LegCfg{bc, ss, std::max(128, 32 * leg_warps((per * js + 31) / 32)), analysis_smem_bytes<Epi>(L, p->nh, bc, ss),
+                dim3(n_pairs(top) * ss, gy)};
 }
 
 inline int row_threads(const aeolus_plan_impl* p) { return p->tune_row_threads > 0 ? p->tune_row_threads : 256; }
@@ -72,8 +99,8 @@ template <class Derive>
 int launch_synth(const aeolus_plan_impl* p, const Derive& d, double2* FG, int nblk, int batch,
                  cudaStream_t st) {
   const LegCfg c = synth_cfg<Derive>(p, batch);
-  LegArgs a{p->lmax, p->nlat, p->nh, batch, c.bc, p->P, p->PT, FG, nblk};
-  auto kern = legendre_synth_kernel<Derive, kSynthCPT>;
+  LegArgs a{p->lmax, p->nlat, p->nh, batch, c.bc, c.ss, p->P, p->PT, FG, nblk};
+  auto kern = legendre_synth_kernel<Derive>;
   int s = allow_smem(kern, c.smem);
   if (s) return s;
   ProfScope prof("legendre_synth_f64", st);
@@ -86,7 +113,7 @@ template <class Epi>
 int launch_analysis(const aeolus_plan_impl* p, const Epi& e, double2* FG, int nblk, int batch,
                     cudaStream_t st) {
   const LegCfg c = analysis_cfg<Epi>(p, batch);
-  LegArgs a{p->lmax, p->nlat, p->nh, batch, c.bc, p->P, p->PT, FG, nblk};
+  LegArgs a{p->lmax, p->nlat, p->nh, batch, c.bc, c.ss, p->P, p->PT, FG, nblk};
   auto kern = legendre_analysis_kernel<Epi>;
   int s = allow_smem(kern, c.smem);
   if (s) return s;
