@@ -104,19 +104,29 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
                        : nullptr;
     void* scratch = static_cast<char*>(work) + align256(fg_bytes(p, NB, batch)) +
                     (split ? align256(fg_bytes(p, Pw::NOUT, batch)) : 0);
-    int s = split ? launch_split_synth(p, d, FG, NB, batch, scratch, st) : launch_synth(p, d, FG, NB, batch, st);
+    // FP64: blocks of the contracted fields (RowSrc), G over the same blocks
+    constexpr int N64 = RowSrc<Pw>::NBLK > Pw::NOUT ? RowSrc<Pw>::NBLK : Pw::NOUT;
+    int s;
+    if (split) {
+      s = launch_split_synth(p, d, FG, NB, batch, scratch, st);
+    } else if constexpr (RowSrc<Pw>::NBLK != Pw::NIN) {
+      s = launch_synth(p, typename Derive::Contracted{d}, FG, N64, batch, st);
+    } else {
+      s = launch_synth(p, d, FG, N64, batch, st);
+    }
     if (s) return s;
     RowArgs ra{};
     ra.batch = batch;
     ra.FG = FG;
-    ra.nblk = NB;
+    ra.nblk = split ? NB : N64;
+    if constexpr (RowSrc<Pw>::NBLK != Pw::NIN) ra.ir = d.s.ir;
     ra.G = G;
     ra.gblk = Pw::NOUT;
     ra.status = status;
     ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
     if ((s = launch_rows<Pw, kInF, kOutG>(p, pw, ra, st))) return s;
     return split ? launch_split_anal(p, e, G, Pw::NOUT, batch, scratch, st)
-                 : launch_analysis(p, e, FG, NB, batch, st);
+                 : launch_analysis(p, e, FG, N64, batch, st);
   }
   const long nc = p->ncol, np = p->npoints;
   char* w = static_cast<char*>(work);

@@ -139,7 +139,6 @@ struct aeolus_plan_impl {
   // per CTA of the FP64 Legendre synthesis / analysis, threads of the row
   // stage, members per CTA of the split-path slicing kernels
   int tune_bc_synth = 0, tune_bc_anal = 0, tune_row_threads = 0, tune_slice_mb = 0, tune_slice_mb_anal = 0;
-  FftInfo fft{};   // FP64 row stage (radix 2..5)
   FftInfo fftx{};  // fixed-point row stage (radix 2..5 and 8, in place)
   // device tables (Gauss)
   double* x = nullptr;       // [nlat] cos(colatitude) = sin(latitude)
@@ -148,7 +147,6 @@ struct aeolus_plan_impl {
   double* fgrid = nullptr;   // [nlat] or [npoints]: synthesis of the unit (1,0) mode
   double* P = nullptr;       // [tri_off(m)*nh + (l-m)*nh + jn]  (row jn fastest)
   double* PT = nullptr;      // [tri_off(m)*nh + jn*(L+1-m) + (l-m)] (degree fastest)
-  double2* tw = nullptr;     // [nlon] exp(-2 pi i q / nlon)
   float4* twdf = nullptr;    // [nlon] the same twiddles as double-float (re.hi, re.lo, im.hi, im.lo)
   FxW* twfx = nullptr;       // [nlon] the same twiddles as Q61 31-bit limbs (fixed-point rows)
   int* fft_irev = nullptr;   // [fftx.n] position of natural index q in digit-reversed order (in-place FFTs)

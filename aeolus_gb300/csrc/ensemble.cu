@@ -67,13 +67,17 @@ struct AnalArg {
   LegArgs a;
   Epi e;
 };
+// FP64 row body of a group: 96-bit transforms with several or one member
+// row per CTA, or direct sums with the twiddles in shared or global memory.
+enum WideRowKind { kWideNR = 0, kWide1, kWideDft, kWideDftG };
 template <class Pw>
 struct RowArg {
   RowArgs a;
   Pw pw;
   const FxW* twfx;
   const float4* twdf;
-  int kind;  // SplitRowKind of the group's plan (split path)
+  int kind;  // SplitRowKind of the group's plan (split path) or WideRowKind (FP64)
+  int gf;    // staged fields of the FP64 direct sums
 };
 template <class Derive>
 struct SliceSynthArg {
@@ -107,10 +111,17 @@ __global__ void __launch_bounds__(256) g_legendre_analysis(Grouped<AnalArg<Epi>>
 }
 
 template <class Pw>
-__global__ void __launch_bounds__(256) g_rows(Grouped<RowArg<Pw>> g) {
+__global__ void __launch_bounds__(kWideMaxThreads, 2) g_rows(Grouped<RowArg<Pw>> g, FxConst kc) {
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
-  row_body<Pw, kInF, kOutG>(g.arg[k].a, g.arg[k].pw, loc % g.gx[k], loc / g.gx[k]);
+  const RowArg<Pw>& r = g.arg[k];
+  const int bx = loc % g.gx[k], by = loc / g.gx[k];
+  switch (r.kind) {
+    case kWideNR: row_w_body<Pw, w_rows_per_cta<Pw>(), kInF, kOutG>(r.a, r.pw, r.twfx, kc, bx, by); break;
+    case kWide1: row_w_body<Pw, 1, kInF, kOutG>(r.a, r.pw, r.twfx, kc, bx, by); break;
+    case kWideDft: row_w_dft_body<Pw, kInF, kOutG, false>(r.a, r.pw, r.twfx, r.gf, bx, by); break;
+    default: row_w_dft_body<Pw, kInF, kOutG, true>(r.a, r.pw, r.twfx, r.gf, bx, by);
+  }
 }
 
 // Each group runs the row body its plan's single-plan chains run
@@ -329,7 +340,9 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
   using Derive = typename M::Derive;
   using Pw = typename M::Pw;
   using Epi = typename M::Epi;
+  using SDerive = typename M::SplitDerive;  // contracted fields
   constexpr int NIN = M::NIN, NOUT = M::NOUT, NB = NIN > NOUT ? NIN : NOUT;
+  constexpr int N64 = RowSrc<Pw>::NBLK > NOUT ? RowSrc<Pw>::NBLK : NOUT;  // FP64 blocks (run_full_chain)
   const int ng = E->ng;
   Derive der[kMaxGroups];
   Pw pws[kMaxGroups];
@@ -353,44 +366,45 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     RowArgs ra{};
     ra.batch = E->batch[k];
     ra.FG = reinterpret_cast<double2*>(chain[k]);
-    ra.nblk = NB;
+    ra.nblk = E->split ? NB : N64;
+    if constexpr (RowSrc<Pw>::NBLK != NIN) ra.ir = der[k].s.ir;
     ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
     if (E->split) {  // compact G blocks after F, as in run_full_chain
       ra.G = reinterpret_cast<double2*>(chain[k] + align256(fg_bytes(p, NB, E->batch[k])));
       ra.gblk = NOUT;
     }
     row_args(p, ra);
-    if (E->split) ra.fft = p->fftx;
-    const int kind = E->split ? split_row_kind(p) : kRowsRuntime;
-    const bool pfa = kind >= kRowsPfa192;
-    grouped_add(gr, RowArg<Pw>{ra, pws[k], p->twfx, p->twdf, kind},
-                pfa ? row_pfa_grid<Pw>(p->nlat, E->batch[k]) : dim3(p->nlat, E->batch[k]));
-    sm_rows = std::max(sm_rows, E->split ? split_row_smem_bytes<Pw>(p) : row_smem_bytes<Pw>(p->fft));
-    row_thr = std::max(row_thr, row_threads(p));
-    if (kind != kRowsRuntime) fixed_thr = true;
+    const WideRowCfg wc = wide_row_cfg<Pw>(p, E->batch[k]);
+    const int kind = E->split ? split_row_kind(p) : !p->fftx.use_fft ? (wc.gtab ? kWideDftG : kWideDft) : wc.nr > 1 ? kWideNR : kWide1;
+    const bool pfa = E->split && kind >= kRowsPfa192;
+    grouped_add(gr, RowArg<Pw>{ra, pws[k], p->twfx, p->twdf, kind, wc.gf},
+                !E->split ? wc.grid : pfa ? row_pfa_grid<Pw>(p->nlat, E->batch[k]) : dim3(p->nlat, E->batch[k]));
+    sm_rows = std::max(sm_rows, E->split ? split_row_smem_bytes<Pw>(p) : wc.smem);
+    row_thr = std::max(row_thr, E->split ? row_threads(p) : wc.threads);
+    if (E->split && kind != kRowsRuntime) fixed_thr = true;
   }
   if (fixed_thr) row_thr = kPfaThreads;
   if (!E->split) {
-    Grouped<SynthArg<Derive>> gs{};
+    Grouped<SynthArg<SDerive>> gs{};
     Grouped<AnalArg<Epi>> ga{};
     size_t sm_s = 0, sm_a = 0;
     int thr_s = 64, thr_a = 64;
     for (int k = 0; k < ng; ++k) {
       const aeolus_plan_impl* p = E->plan[k];
       double2* FG = reinterpret_cast<double2*>(chain[k]);
-      const LegCfg cs = synth_cfg<Derive>(p, E->batch[k]);
+      const LegCfg cs = synth_cfg<SDerive>(p, E->batch[k]);
       const LegCfg ca = analysis_cfg<Epi>(p, E->batch[k]);
-      grouped_add(gs, SynthArg<Derive>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], cs.bc, cs.ss, p->P, p->PT, FG, NB},
-                                       der[k]},
+      grouped_add(gs, SynthArg<SDerive>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], cs.bc, cs.ss, p->P, p->PT, FG, N64},
+                                        M::split_derive(der[k])},
                   cs.grid);
-      grouped_add(ga, AnalArg<Epi>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], ca.bc, ca.ss, p->P, p->PT, FG, NB}, epi[k]},
+      grouped_add(ga, AnalArg<Epi>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], ca.bc, ca.ss, p->P, p->PT, FG, N64}, epi[k]},
                   ca.grid);
       sm_s = std::max(sm_s, cs.smem);
       sm_a = std::max(sm_a, ca.smem);
       thr_s = std::max(thr_s, cs.threads);
       thr_a = std::max(thr_a, ca.threads);
     }
-    auto k1 = g_legendre_synth<Derive>;
+    auto k1 = g_legendre_synth<SDerive>;
     auto k2 = g_rows<Pw>;
     auto k3 = g_legendre_analysis<Epi>;
     if ((s = allow_smem(k1, sm_s)) || (s = allow_smem(k2, sm_rows)) || (s = allow_smem(k3, sm_a))) return s;
@@ -401,7 +415,7 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     }
     {
       ProfScope prof("ens_rows", st);
-      k2<<<gr.start[ng], row_thr, sm_rows, st>>>(gr);
+      k2<<<gr.start[ng], row_thr, sm_rows, st>>>(gr, fx_consts());
       AE_LAUNCH("g_rows");
     }
     ProfScope prof("ens_legendre_analysis_f64", st);
@@ -410,7 +424,6 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     return AEOLUS_OK;
   }
   // split precision
-  using SDerive = typename M::SplitDerive;
   constexpr int NS = SDerive::NF;  // contracted fields
   using SEpi = SynthEpi<NS, SynthOut<SDerive>>;
   Grouped<SliceSynthArg<SDerive>> gss{};

@@ -10,6 +10,7 @@
 #include "rows.cuh"
 #include "rows_fx.cuh"
 #include "rows_pfa.cuh"
+#include "rows_w.cuh"
 
 namespace aeolus {
 
@@ -127,9 +128,8 @@ int launch_analysis(const aeolus_plan_impl* p, const Epi& e, double2* FG, int nb
 inline void row_args(const aeolus_plan_impl* p, RowArgs& a) {
   a.L = p->lmax;
   a.nlat = p->nlat;
-  a.fft = p->fft;
+  a.fft = p->fftx;
   a.irev = p->fft_irev;
-  a.tw = p->tw;
   a.coslat = p->coslat;
   a.fgrid = p->fgrid;
   a.wq = a.unit_weights ? nullptr : p->wq;
@@ -214,15 +214,46 @@ size_t split_row_smem_bytes(const aeolus_plan_impl* p) {
   }
 }
 
+// Launch shape of the FP64 row stage (results do not depend on it).
+struct WideRowCfg {
+  int nr;       // member rows per CTA (FFT lengths)
+  int gf;       // staged fields (direct sums)
+  bool gtab;    // twiddles from global memory (rows too long for a shared table)
+  int threads;
+  size_t smem;
+  dim3 grid;
+};
+template <class Pw>
+WideRowCfg wide_row_cfg(const aeolus_plan_impl* p, int batch) {
+  WideRowCfg c{1, 0, false, 128, 0, dim3(p->nlat, batch)};
+  const FftInfo& f = p->fftx;
+  if (f.use_fft) {
+    constexpr int NR = w_rows_per_cta<Pw>();
+    const long grouped = (long)p->nlat * ((batch + NR - 1) / NR);
+    if (grouped >= 4L * p->sm_count && row_w_smem_bytes<Pw>(f, NR) <= 72 * 1024) {
+      c.nr = NR;
+      c.grid.y = (batch + NR - 1) / NR;
+    }
+    c.smem = row_w_smem_bytes<Pw>(f, c.nr);
+    // few rows: twice the threads shorten each row; otherwise more CTAs per SM
+    if ((long)c.grid.x * c.grid.y <= 2L * p->sm_count) c.threads = 256;
+  } else {
+    c.gf = row_w_dft_group<Pw>(f, p->lmax);
+    c.gtab = row_w_dft_smem<Pw>(f, p->lmax, c.gf, false) > 220 * 1024;
+    c.smem = row_w_dft_smem<Pw>(f, p->lmax, c.gf, c.gtab);
+    const int items = (std::min(c.gf, Pw::NIN) + dft_fields<Pw::NIN>() - 1) / dft_fields<Pw::NIN>() * (f.N / 2 + 1);
+    c.threads = 32 * leg_warps((items + 31) / 32);
+  }
+  if (p->tune_row_threads > 0) c.threads = std::min(p->tune_row_threads, kWideMaxThreads);
+  return c;
+}
+
 template <class Pw, int IN_MODE, int OUT_MODE>
 int launch_rows(const aeolus_plan_impl* p, const Pw& pw, RowArgs a, cudaStream_t st) {
   row_args(p, a);
-  dim3 grid(p->nlat, a.batch);
-  const int threads = row_threads(p);
   if (p->precision == AEOLUS_PREC_SPLIT_BF16) {
     // split-precision path: fixed-point FFTs, double-float products; every
     // row stage gets kernels compiled for the common radix sequences
-    a.fft = p->fftx;
     switch (split_row_kind(p)) {
       case kRowsPfa192: return launch_rows_pfa<Pw, IN_MODE, OUT_MODE, Pfa192>(p, pw, a, st);
       case kRowsPfa160: return launch_rows_pfa<Pw, IN_MODE, OUT_MODE, Pfa160>(p, pw, a, st);
@@ -233,13 +264,17 @@ int launch_rows(const aeolus_plan_impl* p, const Pw& pw, RowArgs a, cudaStream_t
       default: return launch_rows_fx<Pw, IN_MODE, OUT_MODE, FftRuntime>(p, pw, a, st);
     }
   }
-  const size_t sm = row_smem_bytes<Pw>(p->fft);
-  auto kern = row_kernel<Pw, IN_MODE, OUT_MODE>;
-  int s = allow_smem(kern, sm);
+  const WideRowCfg c = wide_row_cfg<Pw>(p, a.batch);
+  const char* name = IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_c2r_products_r2c" : "rows_c2r") : "rows_r2c";
+  constexpr int NR = w_rows_per_cta<Pw>();
+  auto kern = c.nr == 1 ? row_kernel_w<Pw, 1, IN_MODE, OUT_MODE> : row_kernel_w<Pw, NR, IN_MODE, OUT_MODE>;
+  auto kdft = c.gtab ? row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, true> : row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, false>;
+  int s = p->fftx.use_fft ? allow_smem(kern, c.smem) : allow_smem(kdft, c.smem);
   if (s) return s;
-  ProfScope prof(IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_c2r_products_r2c" : "rows_c2r") : "rows_r2c", st);
-  kern<<<grid, threads, sm, st>>>(a, pw);
-  AE_LAUNCH("row_kernel");
+  ProfScope prof(name, st);
+  if (p->fftx.use_fft) kern<<<c.grid, c.threads, c.smem, st>>>(a, pw, p->twfx, fx_consts());
+  else kdft<<<c.grid, c.threads, c.smem, st>>>(a, pw, p->twfx, c.gf);
+  AE_LAUNCH("row_kernel_w");
   return AEOLUS_OK;
 }
 

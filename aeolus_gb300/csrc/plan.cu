@@ -238,7 +238,7 @@ void twiddles(int N, std::vector<double2>& tw) {
   }
 }
 
-void plan_fft(int N, int L, FftInfo& f, bool radix8) {
+void plan_fft(int N, int L, FftInfo& f) {
   std::memset(&f, 0, sizeof(f));
   f.N = N;
   f.n = (N + 1) / 2;
@@ -246,16 +246,16 @@ void plan_fft(int N, int L, FftInfo& f, bool radix8) {
   if (N % 2 != 0) return;
   int n = N / 2;
   if (L > n - 1) return;  // Nyquist / aliased orders: direct DFT handles them
-  // Radix order: odd radices first, then 2 or 4, then 4s (or 8s with
-  // radix8).  A stage with sub-transform length 1 touches shared memory at a
-  // stride of its radix, which is free of bank conflicts for an odd radix.
+  // Radix order: odd radices first, then 2 or 4, then 8s.  A stage with sub-
+  // transform length 1 touches shared memory at a stride of its radix, which
+  // is free of bank conflicts for an odd radix.
   int rem = n, nf = 0, fac[kMaxFactors];
   int c2 = 0;
   while (rem % 2 == 0) { ++c2; rem /= 2; }
   const int odd[2] = {3, 5};
   for (int r : odd)
     while (rem % r == 0 && nf < kMaxFactors) { fac[nf++] = r; rem /= r; }
-  const int big = radix8 ? 3 : 2;  // log2 of the main power-of-two radix
+  const int big = 3;                // log2 of the main power-of-two radix
   const int lead = c2 % big;        // leading radix 2 or 4
   if (lead > 0 && nf < kMaxFactors) fac[nf++] = 1 << lead;
   for (int i = 0; i < c2 / big && nf < kMaxFactors; ++i) fac[nf++] = 1 << big;
@@ -343,7 +343,6 @@ void free_plan(aeolus_plan_impl* p) {
   for (double* b : bufs)
     if (b) cudaFree(b);
   if (p->dcoef_df) cudaFree(p->dcoef_df);
-  if (p->tw) cudaFree(p->tw);
   if (p->twdf) cudaFree(p->twdf);
   if (p->twfx) cudaFree(p->twfx);
   if (p->fft_irev) cudaFree(p->fft_irev);
@@ -450,8 +449,7 @@ extern "C" int aeolus_plan_create_gauss(int nlat, int nlon, int lmax, double rad
   p->radius = radius;
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device);
-  plan_fft(nlon, lmax, p->fft, false);
-  plan_fft(nlon, lmax, p->fftx, true);
+  plan_fft(nlon, lmax, p->fftx);
   int s = AEOLUS_OK;
   auto bail = [&](int st) { free_plan(p); delete p; return st; };
   const int L = lmax, nh = p->nh;
@@ -490,7 +488,6 @@ extern "C" int aeolus_plan_create_gauss(int nlat, int nlon, int lmax, double rad
   if ((s = cuda_check(cudaGetLastError(), "legendre_table_kernel"))) return bail(s);
   std::vector<double2> tw;
   twiddles(nlon, tw);
-  if ((s = cuda_check(cudaMalloc(&p->tw, nlon * sizeof(double2)), "cudaMalloc tw"))) return bail(s);
   {
     std::vector<float4> twf(nlon);
     for (int q = 0; q < nlon; ++q) {
@@ -528,8 +525,6 @@ extern "C" int aeolus_plan_create_gauss(int nlat, int nlon, int lmax, double rad
         return bail(s);
     }
   }
-  if ((s = cuda_check(cudaMemcpy(p->tw, tw.data(), nlon * sizeof(double2), cudaMemcpyHostToDevice), "tw")))
-    return bail(s);
   if ((s = common_tables(p))) return bail(s);
   if ((s = cuda_check(cudaDeviceSynchronize(), "plan build"))) return bail(s);
   *out = p;
