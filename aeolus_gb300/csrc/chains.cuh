@@ -15,6 +15,14 @@ namespace aeolus {
 
 inline unsigned blocks_for(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+template <class Pw>
+void launch_points_pointwise(cudaStream_t st, long np, int batch, const double* in, long in_b, long in_f, double* out,
+                             long out_b, long out_f, const double* coslat, const double* fgrid, const double* w,
+                             unsigned* status, const Pw& pw) {
+  launch_pdl(points_pointwise_kernel<Pw>, dim3(blocks_for(np * batch, 128)), dim3(128), 0, st, np, batch, in, in_b,
+             in_f, out, out_b, out_f, coslat, fgrid, w, status, pw);
+}
+
 // ---------------------------------------------------------------- sizes
 inline bool split_on(const aeolus_plan_impl* p) {
   return p->kind == kGauss && p->precision == AEOLUS_PREC_SPLIT_BF16 && p->split != nullptr;
@@ -140,16 +148,16 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
   w += align256((size_t)batch * Pw::NOUT * nc * 8);
   void* dscratch = w;
   const long nlm = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
-  derive_cols_kernel<Derive><<<blocks_for(nlm, 128), 128, 0, st>>>(p->lmax, batch, nc, V, d);
+  launch_pdl(derive_cols_kernel<Derive>, dim3(blocks_for(nlm, 128)), dim3(128), 0, st, p->lmax, batch, nc, V, d);
   AE_LAUNCH("derive_cols_kernel");
   int s = points_synth(p, V, Gr, batch * Pw::NIN, dscratch, st);
   if (s) return s;
-  points_pointwise_kernel<Pw><<<blocks_for(np * batch, 128), 128, 0, st>>>(
-      np, batch, Gr, (long)Pw::NIN * np, np, Wt, (long)Pw::NOUT * np, np, p->coslat, p->fgrid, p->wpts, status, pw);
+  launch_points_pointwise(st, np, batch, Gr, (long)Pw::NIN * np, np, Wt, (long)Pw::NOUT * np, np, p->coslat, p->fgrid,
+                          p->wpts, status, pw);
   AE_LAUNCH("points_pointwise_kernel");
   if ((s = points_analysis(p, Wt, C, batch * Pw::NOUT, dscratch, st))) return s;
   const long n2 = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
-  epilogue_cols_kernel<Epi><<<blocks_for(n2, 128), 128, 0, st>>>(p->lmax, batch, nc, C, e);
+  launch_pdl(epilogue_cols_kernel<Epi>, dim3(blocks_for(n2, 128)), dim3(128), 0, st, p->lmax, batch, nc, static_cast<const double*>(C), e);
   AE_LAUNCH("epilogue_cols_kernel");
   return AEOLUS_OK;
 }
@@ -183,13 +191,13 @@ int run_synth_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, in
   w += align256((size_t)batch * Pw::NIN * np * 8);
   void* dscratch = w;
   const long nlm = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
-  derive_cols_kernel<Derive><<<blocks_for(nlm, 128), 128, 0, st>>>(p->lmax, batch, nc, V, d);
+  launch_pdl(derive_cols_kernel<Derive>, dim3(blocks_for(nlm, 128)), dim3(128), 0, st, p->lmax, batch, nc, V, d);
   AE_LAUNCH("derive_cols_kernel");
   const bool direct = Pw::kIdentity && out_b == np;
   int s = points_synth(p, V, direct ? out : Gr, batch * Pw::NIN, dscratch, st);
   if (s || direct) return s;
-  points_pointwise_kernel<Pw><<<blocks_for(np * batch, 128), 128, 0, st>>>(
-      np, batch, Gr, (long)Pw::NIN * np, np, out, out_b, out_f, p->coslat, p->fgrid, nullptr, status, pw);
+  launch_points_pointwise(st, np, batch, Gr, (long)Pw::NIN * np, np, out, out_b, out_f, p->coslat, p->fgrid, nullptr,
+                          status, pw);
   AE_LAUNCH("points_pointwise_kernel");
   return AEOLUS_OK;
 }
@@ -225,14 +233,13 @@ int run_anal_chain(const aeolus_plan_impl* p, const Pw& pw, const Epi& e, int ba
   double* C = reinterpret_cast<double*>(w);
   w += align256((size_t)batch * Pw::NOUT * nc * 8);
   void* dscratch = w;
-  points_pointwise_kernel<Pw><<<blocks_for(np * batch, 128), 128, 0, st>>>(
-      np, batch, in, in_b, in_f, Wt, (long)Pw::NOUT * np, np, p->coslat, p->fgrid, unit_weights ? nullptr : p->wpts,
-      nullptr, pw);
+  launch_points_pointwise(st, np, batch, in, in_b, in_f, Wt, (long)Pw::NOUT * np, np, p->coslat, p->fgrid,
+                          unit_weights ? nullptr : p->wpts, nullptr, pw);
   AE_LAUNCH("points_pointwise_kernel");
   int s = points_analysis(p, Wt, C, batch * Pw::NOUT, dscratch, st);
   if (s) return s;
   const long n2 = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
-  epilogue_cols_kernel<Epi><<<blocks_for(n2, 128), 128, 0, st>>>(p->lmax, batch, nc, C, e);
+  launch_pdl(epilogue_cols_kernel<Epi>, dim3(blocks_for(n2, 128)), dim3(128), 0, st, p->lmax, batch, nc, static_cast<const double*>(C), e);
   AE_LAUNCH("epilogue_cols_kernel");
   return AEOLUS_OK;
 }

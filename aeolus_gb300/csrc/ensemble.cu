@@ -98,6 +98,7 @@ struct SliceAnalArg {
 
 template <class Derive>
 __global__ void __launch_bounds__(256) g_legendre_synth(Grouped<SynthArg<Derive>> g) {
+  pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
   legendre_synth_body<Derive>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(256) g_legendre_synth(Grouped<SynthArg<Derive>
 
 template <class Epi>
 __global__ void __launch_bounds__(256) g_legendre_analysis(Grouped<AnalArg<Epi>> g) {
+  pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
   legendre_analysis_body<Epi>(g.arg[k].a, g.arg[k].e, loc % g.gx[k], loc / g.gx[k]);
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(256) g_legendre_analysis(Grouped<AnalArg<Epi>>
 
 template <class Pw>
 __global__ void __launch_bounds__(kWideMaxThreads, 2) g_rows(Grouped<RowArg<Pw>> g, FxConst kc) {
+  pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
   const RowArg<Pw>& r = g.arg[k];
@@ -136,7 +139,6 @@ __global__ void __launch_bounds__(kWideMaxThreads, 2) g_rows(Grouped<RowArg<Pw>>
 template <class Pw, bool TH128>
 __global__ void __launch_bounds__(TH128 ? kPfaThreads : 256, TH128 ? 7 : 3)
     g_rows_fx(Grouped<RowArg<Pw>> g, FxConst kc) {
-  pdl_trigger();
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
@@ -155,7 +157,6 @@ __global__ void __launch_bounds__(TH128 ? kPfaThreads : 256, TH128 ? 7 : 3)
 
 template <class Derive>
 __global__ void __launch_bounds__(256) g_slice_synth(Grouped<SliceSynthArg<Derive>> g) {
-  pdl_trigger();
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
@@ -166,7 +167,6 @@ __global__ void __launch_bounds__(256) g_slice_synth(Grouped<SliceSynthArg<Deriv
 
 template <int NF>
 __global__ void __launch_bounds__(256) g_slice_anal(Grouped<SliceAnalArg> g) {
-  pdl_trigger();
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
@@ -410,16 +410,16 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     if ((s = allow_smem(k1, sm_s)) || (s = allow_smem(k2, sm_rows)) || (s = allow_smem(k3, sm_a))) return s;
     {
       ProfScope prof("ens_legendre_synth_f64", st);
-      k1<<<gs.start[ng], thr_s, sm_s, st>>>(gs);
+      launch_pdl(k1, dim3(gs.start[ng]), dim3(thr_s), sm_s, st, gs);
       AE_LAUNCH("g_legendre_synth");
     }
     {
       ProfScope prof("ens_rows", st);
-      k2<<<gr.start[ng], row_thr, sm_rows, st>>>(gr, fx_consts());
+      launch_pdl(k2, dim3(gr.start[ng]), dim3(row_thr), sm_rows, st, gr, fx_consts());
       AE_LAUNCH("g_rows");
     }
     ProfScope prof("ens_legendre_analysis_f64", st);
-    k3<<<ga.start[ng], thr_a, sm_a, st>>>(ga);
+    launch_pdl(k3, dim3(ga.start[ng]), dim3(thr_a), sm_a, st, ga);
     AE_LAUNCH("g_legendre_analysis");
     return AEOLUS_OK;
   }

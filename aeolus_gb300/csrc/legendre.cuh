@@ -128,6 +128,7 @@ __device__ __forceinline__ void legendre_synth_body(const LegArgs& a, const Deri
 
 template <class Derive>
 __global__ void __launch_bounds__(256) legendre_synth_kernel(LegArgs a, Derive d) {
+  pdl_wait();
   legendre_synth_body<Derive>(a, d, blockIdx.x, blockIdx.y);
 }
 
@@ -246,6 +247,7 @@ __device__ __forceinline__ void legendre_analysis_body(const LegArgs& a, const E
 
 template <class Epi>
 __global__ void __launch_bounds__(256) legendre_analysis_kernel(LegArgs a, Epi e) {
+  pdl_wait();
   legendre_analysis_body<Epi>(a, e, blockIdx.x, blockIdx.y);
 }
 

@@ -105,7 +105,7 @@ int launch_synth(const aeolus_plan_impl* p, const Derive& d, double2* FG, int nb
   int s = allow_smem(kern, c.smem);
   if (s) return s;
   ProfScope prof("legendre_synth_f64", st);
-  kern<<<c.grid, c.threads, c.smem, st>>>(a, d);
+  launch_pdl(kern, c.grid, dim3(c.threads), c.smem, st, a, d);
   AE_LAUNCH("legendre_synth_kernel");
   return AEOLUS_OK;
 }
@@ -119,7 +119,7 @@ int launch_analysis(const aeolus_plan_impl* p, const Epi& e, double2* FG, int nb
   int s = allow_smem(kern, c.smem);
   if (s) return s;
   ProfScope prof("legendre_analysis_f64", st);
-  kern<<<c.grid, c.threads, c.smem, st>>>(a, e);
+  launch_pdl(kern, c.grid, dim3(c.threads), c.smem, st, a, e);
   AE_LAUNCH("legendre_analysis_kernel");
   return AEOLUS_OK;
 }
@@ -143,7 +143,8 @@ int launch_rows_fx(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, cu
   if (s) return s;
   ProfScope prof(IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_fx_c2r_products_r2c" : "rows_fx_c2r") : "rows_fx_r2c",
                  st);
-  kern<<<dim3(p->nlat, a.batch), row_threads(p), sm, st>>>(a, pw, p->twfx, p->twdf, fx_consts());
+  launch_pdl(kern, dim3(p->nlat, a.batch), dim3(row_threads(p)), sm, st, a, pw, static_cast<const FxW*>(p->twfx),
+             static_cast<const float4*>(p->twdf), fx_consts());
   AE_LAUNCH("row_kernel_fx");
   return AEOLUS_OK;
 }
@@ -158,7 +159,8 @@ int launch_rows_fx8(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, c
   if (s) return s;
   ProfScope prof(IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_fx_c2r_products_r2c" : "rows_fx_c2r") : "rows_fx_r2c",
                  st);
-  kern<<<dim3(p->nlat, a.batch), kFx8Threads, sm, st>>>(a, pw, p->twfx, fx_consts());
+  launch_pdl(kern, dim3(p->nlat, a.batch), dim3(kFx8Threads), sm, st, a, pw, static_cast<const FxW*>(p->twfx),
+             fx_consts());
   AE_LAUNCH("row_kernel_fx8");
   return AEOLUS_OK;
 }
@@ -272,8 +274,9 @@ int launch_rows(const aeolus_plan_impl* p, const Pw& pw, RowArgs a, cudaStream_t
   int s = p->fftx.use_fft ? allow_smem(kern, c.smem) : allow_smem(kdft, c.smem);
   if (s) return s;
   ProfScope prof(name, st);
-  if (p->fftx.use_fft) kern<<<c.grid, c.threads, c.smem, st>>>(a, pw, p->twfx, fx_consts());
-  else kdft<<<c.grid, c.threads, c.smem, st>>>(a, pw, p->twfx, c.gf);
+  const FxW* tw = p->twfx;
+  if (p->fftx.use_fft) launch_pdl(kern, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, fx_consts());
+  else launch_pdl(kdft, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, c.gf);
   AE_LAUNCH("row_kernel_w");
   return AEOLUS_OK;
 }

@@ -70,7 +70,7 @@ namespace {
 template <int NT>
 void synth_pass(long M, int K, int N, const double* B, const double* V, double* out, cudaStream_t st) {
   const long grid = (M + kPtRows - 1) / kPtRows * ((N + NT - 1) / NT);
-  points_synth_kernel<NT><<<(unsigned)grid, kPtThreads, 0, st>>>(M, K, N, B, V, out);
+  launch_pdl(points_synth_kernel<NT>, dim3((unsigned)grid), dim3(kPtThreads), 0, st, M, K, N, B, V, out);
 }
 
 // Four basis columns per CTA share each point's data values once there are
@@ -80,9 +80,9 @@ template <int NT>
 void analysis_pass(int M, long K, int N, const double* B, const double* W, double* C, int sm_count, cudaStream_t st) {
   const long passes = (N + NT - 1) / NT;
   if (M >= 16 * sm_count)
-    points_analysis_kernel<NT, 4><<<(unsigned)((M + 3) / 4 * passes), kPtThreads, 0, st>>>(M, K, N, B, W, C);
+    launch_pdl(points_analysis_kernel<NT, 4>, dim3((unsigned)((M + 3) / 4 * passes)), dim3(kPtThreads), 0, st, M, K, N, B, W, C);
   else
-    points_analysis_kernel<NT, 1><<<(unsigned)(M * passes), kPtThreads, 0, st>>>(M, K, N, B, W, C);
+    launch_pdl(points_analysis_kernel<NT, 1>, dim3((unsigned)(M * passes)), dim3(kPtThreads), 0, st, M, K, N, B, W, C);
 }
 
 inline int pass_columns(int N) {

@@ -22,6 +22,7 @@ __host__ __device__ inline long col_sin(int l, int m, int L) { return col_base(m
 // the dense square, orders fastest: coalesced reads, no search for the order).
 template <class Derive>
 __global__ void derive_cols_kernel(int L, int batch, long ncol, double* __restrict__ V, Derive d) {
+  pdl_wait();
   constexpr int NF = Derive::NF;
   const long n2 = (long)(L + 1) * (L + 1);
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -52,6 +53,7 @@ __global__ void points_pointwise_kernel(long npts, int batch, const double* __re
                                         double* __restrict__ Out, long out_b, long out_f,
                                         const double* __restrict__ coslat, const double* __restrict__ fgrid,
                                         const double* __restrict__ w, unsigned* status, Pw pw) {
+  pdl_wait();
   constexpr int NIN = Pw::NIN, NOUT = Pw::NOUT;
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= npts * batch) return;
@@ -59,7 +61,7 @@ __global__ void points_pointwise_kernel(long npts, int batch, const double* __re
   const long p = idx - (long)b * npts;
   double in[NIN], out[NOUT];
 #pragma unroll
-  for (int f = 0; f < NIN; ++f) in[f] = Gr[(long)b * in_b + (long)f * in_f + p];
+  for (int f = 0; f < NIN; ++f) in[f] = __ldcg(Gr + (long)b * in_b + (long)f * in_f + p);
   const unsigned bits = pw(coslat[p], fgrid[p], in, out);
   if (status && bits) atomicOr(&status[b], bits);
   const double sc = w ? w[p] : 1.0;
@@ -70,6 +72,7 @@ __global__ void points_pointwise_kernel(long npts, int batch, const double* __re
 // a_lm from real analysis columns; one thread per (b, l, m) of the dense square.
 template <class Epi>
 __global__ void epilogue_cols_kernel(int L, int batch, long ncol, const double* __restrict__ C, Epi e) {
+  pdl_wait();
   constexpr int NF = Epi::NF;
   const long n2 = (long)(L + 1) * (L + 1);
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,7 +88,7 @@ __global__ void epilogue_cols_kernel(int L, int batch, long ncol, const double* 
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
     const double* col = C + ((long)b * NF + f) * ncol;
-    acc[f] = make_double2(col[col_cos(l, m, L)], m == 0 ? 0.0 : -col[col_sin(l, m, L)]);
+    acc[f] = make_double2(__ldcg(col + col_cos(l, m, L)), m == 0 ? 0.0 : -__ldcg(col + col_sin(l, m, L)));
   }
   e.finish(b, l, m, acc);
 }
@@ -114,6 +117,7 @@ template <int NT>
 __global__ void __launch_bounds__(kPtThreads) points_synth_kernel(long M, int K, int N, const double* __restrict__ B,
                                                                   const double* __restrict__ V,
                                                                   double* __restrict__ out) {
+  pdl_wait();
   __shared__ double sV[kPtChunk][NT];
   __shared__ double sR[kPtThreads / 32][kPtRows][NT];
   const unsigned rb = (unsigned)((M + kPtRows - 1) / kPtRows);  // row blocks; passes are the slow grid index
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(kPtThreads) points_synth_kernel(long M, int K,
     __syncthreads();
     for (int e = threadIdx.x; e < NT * kPtChunk; e += kPtThreads) {
       const int k = e % kPtChunk, q = e / kPtChunk;
-      if (k < kn) sV[k][q] = q < nn ? V[(long)(n0 + q) * K + k0 + k] : 0.0;
+      if (k < kn) sV[k][q] = q < nn ? __ldcg(V + (long)(n0 + q) * K + k0 + k) : 0.0;
     }
     __syncthreads();
 #pragma unroll 8
@@ -163,6 +167,7 @@ template <int NT, int CT>
 __global__ void __launch_bounds__(kPtThreads) points_analysis_kernel(int M, long K, int N, const double* __restrict__ B,
                                                                      const double* __restrict__ W,
                                                                      double* __restrict__ C) {
+  pdl_wait();
   __shared__ double sR[kPtThreads / 32][CT * NT];
   const unsigned cb = (unsigned)((M + CT - 1) / CT);
   const int n0 = (int)(blockIdx.x / cb) * NT, nn = min(NT, N - n0);
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(kPtThreads) points_analysis_kernel(int M, long
 #pragma unroll
     for (int i = 0; i < CT; ++i) b[i] = __ldg(Bc[i] + p);
 #pragma unroll
-    for (int q = 0; q < NT; ++q) w[q] = __ldg(Wn[q] + p);
+    for (int q = 0; q < NT; ++q) w[q] = __ldcg(Wn[q] + p);
 #pragma unroll
     for (int i = 0; i < CT; ++i)
 #pragma unroll

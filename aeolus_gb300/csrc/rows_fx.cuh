@@ -793,6 +793,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
 template <class Pw, int IN_MODE, int OUT_MODE, int R0>
 __global__ void __launch_bounds__(kFx8Threads, 6) row_kernel_fx8(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                  FxConst kc) {
+  pdl_wait();
   row_fx8_body<Pw, IN_MODE, OUT_MODE, R0>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
 }
 
@@ -813,6 +814,7 @@ inline size_t row_fx_smem_bytes(const FftInfo& f) {
 template <class Pw, int IN_MODE, int OUT_MODE, class FFT>
 __global__ void __launch_bounds__(256, 3) row_kernel_fx(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                      const float4* __restrict__ twdf, FxConst kc) {
+  pdl_wait();
   row_fx_body<Pw, IN_MODE, OUT_MODE, FFT>(a, pw, twfx, twdf, kc, blockIdx.x, blockIdx.y);
 }
 

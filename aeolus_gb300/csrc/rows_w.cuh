@@ -745,11 +745,13 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
 template <class Pw, int NR, int IN_MODE, int OUT_MODE>
 __global__ void __launch_bounds__(kWideMaxThreads, 2) row_kernel_w(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                    FxConst kc) {
+  pdl_wait();
   row_w_body<Pw, NR, IN_MODE, OUT_MODE>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
 }
 template <class Pw, int IN_MODE, int OUT_MODE, bool GTAB>
 __global__ void __launch_bounds__(kWideMaxThreads, 2) row_kernel_w_dft(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                        int gf) {
+  pdl_wait();
   row_w_dft_body<Pw, IN_MODE, OUT_MODE, GTAB>(a, pw, twfx, gf, blockIdx.x, blockIdx.y);
 }
 

@@ -364,7 +364,6 @@ __global__ void __launch_bounds__(256, DeriveHasDf<Derive>::value ? 3 : 4) split
                                                                int batch, int mb, Derive der,
                                                                __nv_bfloat16* __restrict__ dsyn,
                                                                int* __restrict__ ecol) {
-  pdl_trigger();
   pdl_wait();
   split_synth_slice_body<Derive>(dm, kcum, batch, mb, der, dsyn, ecol, blockIdx.x, blockIdx.y, gridDim.y);
 }
@@ -438,7 +437,6 @@ __global__ void __launch_bounds__(kAnalSliceThreads, 8) split_anal_slice_kernel(
                                                               const long long* __restrict__ FG,
                                                               __nv_bfloat16* __restrict__ dana,
                                                               int* __restrict__ ecol) {
-  pdl_trigger();
   pdl_wait();
   split_anal_slice_body<NF>(dm, batch, mb, nblk, FG, dana, ecol, blockIdx.x, blockIdx.y, gridDim.y);
 }
@@ -588,7 +586,6 @@ __global__ void __launch_bounds__(tc_threads<Epi>(), 1) tc_persistent_kernel(Sch
   tc::fence_after_sync();
   const uint32_t tmem = *sm.tmem_slot;
   const int ntiles = sc.count();
-  pdl_trigger();
   pdl_wait();  // global memory only from here on
 
   if (warp == 0) {
@@ -802,7 +799,7 @@ struct SynthEpi {
     const int* ec = ecol + (long long)m * dm.ntiles * kNT + tile * kNT + c0;
     Pre p;
 #pragma unroll
-    for (int i = 0; i < kCols; ++i) p.e[i] = Ej + __ldg(ec + i) - kOut;
+    for (int i = 0; i < kCols; ++i) p.e[i] = Ej + ec[i] - kOut;
     return p;
   }
   template <class Rel>
@@ -896,7 +893,7 @@ struct AnalEpi {
     const int Et = eana[rt * 128 + row];
     const int* ec = ecol + (long long)m * dm.ntiles * kNT + tile * kNT + c0;
 #pragma unroll
-    for (int i = 0; i < kCols; ++i) st.e[i] = Et + __ldg(ec + i) - kOut;
+    for (int i = 0; i < kCols; ++i) st.e[i] = Et + ec[i] - kOut;
   }
   __device__ void seg_add(State& st, uint32_t tbuf, int q, int c0) const {
     float acc[kCols][kAccs];
