@@ -72,6 +72,11 @@ SIGNATURES = {
                                   c_void_p]),
     "aeolus_pe_spectral": (c_int, [c_int, POINTER(PeParams), c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_int, c_void_p]),
+    "aeolus_pe_workspace_bytes": (c_int, [c_void_p, c_int, c_int, POINTER(c_size_t), POINTER(c_size_t)]),
+    "aeolus_pe_tendency": (c_int, [c_void_p, POINTER(PeParams), c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                   c_void_p, c_size_t, c_void_p]),
+    "aeolus_pe_rk4": (c_int, [c_void_p, POINTER(PeParams), c_int, c_void_p, c_void_p, c_void_p, c_int, c_double, c_int,
+                              c_void_p, c_size_t, c_void_p]),
     "aeolus_geodesic_sizes": (c_int, [c_int, POINTER(c_long), POINTER(c_long), POINTER(c_size_t)]),
     "aeolus_geodesic_build": (c_int, [c_int, c_double, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_size_t, c_void_p]),

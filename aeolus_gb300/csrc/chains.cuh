@@ -162,26 +162,37 @@ int run_full_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, con
   return AEOLUS_OK;
 }
 
-// Output grid: out[b * out_b + f * out_f + point].
-template <class Derive, class Pw>
+// Output grid: out[b * out_b + f * out_f + point].  OUT: kOutGrid, or
+// kOutGridDf (double-floats in place of FP64 values; split Gauss plans).
+template <class Derive, class Pw, int OUT = kOutGrid>
 int run_synth_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, int batch, double* out, long out_b,
                     long out_f, void* work, unsigned* status, cudaStream_t st) {
   static_assert(Derive::NF == Pw::NIN, "derive/pointwise field count");
+  constexpr bool kContract = RowSrc<Pw>::NBLK != Pw::NIN;  // longitude derivatives formed after the contraction
   if (p->kind == kGauss) {
     double2* FG = static_cast<double2*>(work);
     void* scratch = static_cast<char*>(work) + align256(fg_bytes(p, Pw::NIN, batch));
-    int s = split_on(p) ? launch_split_synth(p, d, FG, Pw::NIN, batch, scratch, st)
-                        : launch_synth(p, d, FG, Pw::NIN, batch, st);
+    const bool split = split_on(p);
+    int s;
+    if constexpr (kContract) {
+      const typename Derive::Contracted c{d};
+      s = split ? launch_split_synth(p, c, FG, Pw::NIN, batch, scratch, st)
+                : launch_synth(p, c, FG, RowSrc<Pw>::NBLK, batch, st);
+    } else {
+      s = split ? launch_split_synth(p, d, FG, Pw::NIN, batch, scratch, st)
+                : launch_synth(p, d, FG, Pw::NIN, batch, st);
+    }
     if (s) return s;
     RowArgs ra{};
     ra.batch = batch;
     ra.FG = FG;
-    ra.nblk = Pw::NIN;
+    ra.nblk = split ? Pw::NIN : RowSrc<Pw>::NBLK;
+    if constexpr (kContract) ra.ir = d.s.ir;
     ra.gout = out;
     ra.gout_b = out_b;
     ra.gout_f = out_f;
     ra.status = status;
-    return launch_rows<Pw, kInF, kOutGrid>(p, pw, ra, st);
+    return launch_rows<Pw, kInF, OUT>(p, pw, ra, st);
   }
   const long nc = p->ncol, np = p->npoints;
   char* w = static_cast<char*>(work);
@@ -193,7 +204,7 @@ int run_synth_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, in
   const long nlm = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
   launch_pdl(derive_cols_kernel<Derive>, dim3(blocks_for(nlm, 128)), dim3(128), 0, st, p->lmax, batch, nc, V, d);
   AE_LAUNCH("derive_cols_kernel");
-  const bool direct = Pw::kIdentity && out_b == np;
+  const bool direct = Pw::kIdentity && out_f == np && out_b == Pw::NIN * np;
   int s = points_synth(p, V, direct ? out : Gr, batch * Pw::NIN, dscratch, st);
   if (s || direct) return s;
   launch_points_pointwise(st, np, batch, Gr, (long)Pw::NIN * np, np, out, out_b, out_f, p->coslat, p->fgrid, nullptr,
@@ -204,7 +215,7 @@ int run_synth_chain(const aeolus_plan_impl* p, const Derive& d, const Pw& pw, in
 
 // Input grid: in[b * in_b + f * in_f + point].  unit_weights drops the
 // quadrature weights (the transpose of synthesis instead of the analysis).
-template <class Pw, class Epi>
+template <class Pw, class Epi, int IN = kInGrid>
 int run_anal_chain(const aeolus_plan_impl* p, const Pw& pw, const Epi& e, int batch, const double* in, long in_b,
                    long in_f, void* work, cudaStream_t st, bool unit_weights = false) {
   static_assert(Pw::NOUT == Epi::NF, "pointwise/epilogue field count");
@@ -218,7 +229,8 @@ int run_anal_chain(const aeolus_plan_impl* p, const Pw& pw, const Epi& e, int ba
     ra.gin_b = in_b;
     ra.gin_f = in_f;
     ra.unit_weights = unit_weights ? 1 : 0;
-    int s = launch_rows<Pw, kInGrid, kOutG>(p, pw, ra, st);
+    ra.drop = p->lmax - EpiTop<Epi>::top(p->lmax);
+    int s = launch_rows<Pw, IN, kOutG>(p, pw, ra, st);
     if (s) return s;
     if (split_on(p)) {
       void* scratch = static_cast<char*>(work) + align256(fg_bytes(p, Pw::NOUT, batch));

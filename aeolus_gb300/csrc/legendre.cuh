@@ -34,6 +34,12 @@ template <class E>
 struct EpiTop<E, std::enable_if_t<E::kCut>> {
   __host__ __device__ static int top(int L) { return (2 * L) / 3; }
 };
+// kCutPlus: one degree more, which the weak-form curl and divergence of the
+// degrees up to the cut read.
+template <class E>
+struct EpiTop<E, std::enable_if_t<E::kCutPlus>> {
+  __host__ __device__ static int top(int L) { return (2 * L) / 3 + 1 < L ? (2 * L) / 3 + 1 : L; }
+};
 
 struct LegArgs {
   int L, nlat, nh, batch, bc;

@@ -19,6 +19,8 @@
 //   aeolus_pe_spectral  spectral: 2/3 cuts, Simmons-Burridge geopotential of
 //                       the spectral T, -lap(KE + Phi), l = 0 rows of the
 //                       momentum tendencies pinned.
+#include <type_traits>
+
 #include "models.cuh"
 
 namespace aeolus {
@@ -452,6 +454,495 @@ __global__ void pe_spectral_kernel(PeSigma sg, int L, double R, double r_dry, in
   O[(long)3 * K * n2] = keep ? A[(long)kPeOutFields * K * n2] : zero;
 }
 
+// --------------------------------------------------------------------------
+// The whole tendency as one chain (aeolus_pe_tendency, aeolus_pe_rk4): the
+// spectra of a member's K levels and ln p_s go through the transforms as
+// K + 1 "levels" of the batch,
+//   synthesis of 7 contracted fields per level (U, V, zeta, delta, T and the
+//   latitude derivatives of T and eta; the longitude derivatives are formed
+//   from the T and zeta order spectra, and eta = zeta + f on the grid),
+//   column physics, analysis of 6 fields per level (the four integrands and
+//   Z / cos, whose curl and divergence below the 2/3 cut read one degree
+//   more than the cut, not one more than l_max), spectral kernel.
+// Level K carries ln p_s in the T slot (its other fields are zero) and
+// d ln p_s / dt in the first integrand.  Against the composition of the single
+// calls (10 K + 2 fields synthesised, 6 K + 1 analysed to l_max + 1, FP64 grids
+// between the kernels, 14 launches through Python): one FP64 RK4 step at 64 x
+// 128, l_max 42, 8 levels 1.45 -> 0.27 ms; the split tendency of 4 members at
+// 192 x 384, l_max 127, 20 levels 2.13 -> 1.51 ms (columns 376 -> 262 us, bound
+// by instruction issue; 110 us of it are the DRAM bytes).
+constexpr int kPeGrid = 9;  // U, V, zeta, delta, T, T_lam, T_snt, eta_lam, eta_snt
+constexpr int kPeProd = 6;  // the four integrands of kPeOutFields, Z_east / cos, Z_north / cos
+
+struct PeDerive7;
+struct PeDerive {  // every grid field (point-set plans)
+  static constexpr int NF = kPeGrid;
+  using Contracted = PeDerive7;
+  Spec s;
+  const double2* state;
+  int K;
+  double f10;
+  struct Level {
+    const double2 *z, *d, *T;  // null: the level of ln p_s
+  };
+  __device__ Level level(int bk) const {
+    const long n2 = (long)(s.L + 1) * (s.L + 1);
+    const int b = bk / (K + 1), k = bk - b * (K + 1);
+    const double2* S = state + (long)b * (3 * K + 1) * n2;
+    if (k == K) return Level{nullptr, nullptr, S + 3 * K * n2};
+    return Level{S + k * n2, S + (K + k) * n2, S + (2 * K + k) * n2};
+  }
+  __device__ void column(int bk, int l, int m, double2* v) const {
+    const Level f = level(bk);
+    const int L = s.L;
+    const long r = (long)l * (L + 1) + m;
+    const bool lo = l >= 1 && l - 1 >= m, hi = l + 1 <= L;
+    const double2 zero = make_double2(0.0, 0.0);
+    // 1/R C+_{l-1} / lap, 1/R C-_{l+1} / lap, m/R / lap, then the same without 1 / lap
+    double A1, A2, A3, B1, B2, B3;
+    if (s.dcoef) {
+      const double* c = s.dcoef + r * 8;
+      A1 = c[0], A2 = c[1], A3 = c[2], B1 = c[3], B2 = c[4], B3 = c[5];
+    } else {
+      auto il = [&](int ll) { return ll <= 0 ? 0.0 : (s.invlap ? s.invlap[ll] : 1.0 / s.lap(ll)); };
+      B1 = lo ? s.ir * s.cplus[r - (L + 1)] : 0.0;
+      B2 = hi ? s.ir * s.cminus[r + (L + 1)] : 0.0;
+      B3 = (double)m * s.ir;
+      A1 = lo ? B1 * il(l - 1) : 0.0;
+      A2 = hi ? B2 * il(l + 1) : 0.0;
+      A3 = B3 * il(l);
+    }
+    auto at = [&](const double2* a, int off) { return a[r + off * (L + 1)]; };
+    const double2 Tl = f.T[r], T_lo = lo ? at(f.T, -1) : zero, T_hi = hi ? at(f.T, 1) : zero;
+    v[4] = Tl;
+    v[5] = make_double2(-B3 * Tl.y, B3 * Tl.x);
+    v[6] = make_double2(fma(B1, T_lo.x, B2 * T_hi.x), fma(B1, T_lo.y, B2 * T_hi.y));
+    if (!f.z) {
+      v[0] = v[1] = v[2] = v[3] = v[4] = v[7] = v[8] = zero;
+      v[4] = Tl;
+      return;
+    }
+    const double2 zl = f.z[r], dl = f.d[r];
+    double2 z_lo = lo ? at(f.z, -1) : zero, z_hi = hi ? at(f.z, 1) : zero;
+    const double2 d_lo = lo ? at(f.d, -1) : zero, d_hi = hi ? at(f.d, 1) : zero;
+    v[0] = make_double2(fma(A1, z_lo.x, fma(A2, z_hi.x, -A3 * dl.y)), fma(A1, z_lo.y, fma(A2, z_hi.y, A3 * dl.x)));
+    v[1] = make_double2(-fma(A1, d_lo.x, fma(A2, d_hi.x, A3 * zl.y)), fma(A3, zl.x, -fma(A1, d_lo.y, A2 * d_hi.y)));
+    v[2] = zl;
+    v[3] = dl;
+    v[7] = make_double2(-B3 * zl.y, B3 * zl.x);  // f has m = 0: no longitude derivative
+    if (m == 0) {                                // planetary vorticity of the (1, 0) mode in eta
+      if (l - 1 == 1) z_lo.x += f10;
+      if (l + 1 == 1) z_hi.x += f10;
+    }
+    v[8] = make_double2(fma(B1, z_lo.x, B2 * z_hi.x), fma(B1, z_lo.y, B2 * z_hi.y));
+  }
+};
+
+struct PeDerive7 {  // the contracted fields of a Gauss plan
+  static constexpr int NF = 7;
+  static constexpr bool kColumnDf = true;
+  static constexpr int NBLK = kPeGrid;
+  __host__ __device__ static constexpr int blk(int f) { return f < 5 ? f : f == 5 ? 6 : 8; }
+  __host__ __device__ static constexpr int lam_blk(int f) { return f == 4 ? 5 : f == 2 ? 7 : -1; }
+  PeDerive d9;
+  double lam_ir() const { return d9.s.ir; }
+  __device__ void column(int bk, int l, int m, double2* v) const {
+    double2 w[kPeGrid];
+    d9.column(bk, l, m, w);
+#pragma unroll
+    for (int f = 0; f < 5; ++f) v[f] = w[f];
+    v[5] = w[6];
+    v[6] = w[8];
+  }
+  // The same fields in double-float (lanes re, im), as SweDerive7::column_df.
+  __device__ void column_df(int bk, int l, int m, df2* v) const {
+    const Spec& s = d9.s;
+    if (!s.dcoef_df) {
+      double2 w[NF];
+      column(bk, l, m, w);
+#pragma unroll
+      for (int f = 0; f < NF; ++f) v[f] = df2_of_f64x2(w[f]);
+      return;
+    }
+    const PeDerive::Level f = d9.level(bk);
+    const int L = s.L;
+    const long r = (long)l * (L + 1) + m;
+    const float2* c = s.dcoef_df + r * 8;
+    auto k = [&](int i) { return df2_splat(df{c[i].x, c[i].y}); };
+    const bool lo = l >= 1 && l - 1 >= m, hi = l + 1 <= L;
+    const df2 zero = df2{0ull, 0ull};
+    auto at = [&](const double2* a, int off, bool in) { return in ? df2_of_f64x2(a[r + off * (L + 1)]) : zero; };
+    const df2 B1 = k(3), B2 = k(4);
+    v[4] = at(f.T, 0, true);
+    v[5] = df2_add_fast(df2_mul(B1, at(f.T, -1, lo)), df2_mul(B2, at(f.T, 1, hi)));
+    if (!f.z) {
+      v[0] = v[1] = v[2] = v[3] = v[6] = zero;
+      return;
+    }
+    const df2 zl = at(f.z, 0, true), dl = at(f.d, 0, true), d_lo = at(f.d, -1, lo), d_hi = at(f.d, 1, hi);
+    df2 z_lo = at(f.z, -1, lo), z_hi = at(f.z, 1, hi);
+    const df2 A1 = k(0), A2 = k(1), A3 = k(2);
+    v[0] = df2_add_fast(df2_add_fast(df2_mul(A1, z_lo), df2_mul(A2, z_hi)), df2_mul(A3, df2_times_i(dl)));
+    v[1] = df2_sub_fast(df2_mul(A3, df2_times_i(zl)), df2_add_fast(df2_mul(A1, d_lo), df2_mul(A2, d_hi)));
+    v[2] = zl;
+    v[3] = dl;
+    if (m == 0 && (l == 2 || l == 0)) {  // planetary vorticity of the (1, 0) mode in eta
+      df re, im;
+      df2_unpack(l == 2 ? z_lo : z_hi, re, im);
+      re = df_add(re, df_of_f64(d9.f10));
+      (l == 2 ? z_lo : z_hi) = df2_pack(re, im);
+    }
+    v[6] = df2_add_fast(df2_mul(B1, z_lo), df2_mul(B2, z_hi));
+  }
+};
+
+// Identity of N fields.
+template <int N>
+struct PwCopyN {
+  static constexpr int NIN = N, NOUT = N;
+  static constexpr bool kIdentity = true;
+  __device__ unsigned operator()(double, double, const double* in, double* out) const {
+#pragma unroll
+    for (int f = 0; f < N; ++f) out[f] = in[f];
+    return 0u;
+  }
+  __device__ RowDf df_row(double c, double) const { return RowDf{df{0.f, 0.f}, df{0.f, 0.f}, (float)c}; }
+  __device__ unsigned df_op(const RowDf&, const df* in, df* out) const {
+#pragma unroll
+    for (int f = 0; f < N; ++f) out[f] = in[f];
+    return 0u;
+  }
+  __device__ unsigned df_op2(const RowDf&, const df2* in, df2* out) const {
+#pragma unroll
+    for (int f = 0; f < N; ++f) out[f] = in[f];
+    return 0u;
+  }
+};
+struct PePw : PwCopyN<kPeGrid> {  // grid fields; FP64 Gauss plans: T_lam, eta_lam from T, zeta (RowSrc)
+  static constexpr int NBLK64 = 7;
+  __device__ static constexpr int src64(int f) {
+    constexpr int b[kPeGrid] = {0, 1, 2, 3, 4, 4, 5, 2, 6};
+    return b[f];
+  }
+  __device__ static constexpr bool lam64(int f) { return f == 5 || f == 7; }
+};
+
+// Analysed fields of a level, [bk][kPeProd][L+1][L+1]: only the triangle the
+// spectral kernel reads is written.
+struct PeEpi {
+  static constexpr int NF = kPeProd;
+  static constexpr bool kCutPlus = true;
+  double2* out;
+  int L;
+  __device__ void finish_field(int bk, int f, int l, int m, double2 a) const {
+    if (l <= EpiTop<PeEpi>::top(L)) out[(((long)bk * NF + f) * (L + 1) + l) * (L + 1) + m] = a;
+  }
+  __device__ void finish(int bk, int l, int m, const double2* acc) const {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) finish_field(bk, f, l, m, acc[f]);
+  }
+  __device__ void zero(int, int, int) const {}
+};
+
+// Arithmetic of the column kernel: FP64, or double-float on split-precision
+// plans (whose transforms carry ~48 bits).
+__device__ __forceinline__ double pe_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ double pe_add(double a, double b) { return a + b; }
+__device__ __forceinline__ double pe_sub(double a, double b) { return a - b; }
+__device__ __forceinline__ double pe_neg(double a) { return -a; }
+__device__ __forceinline__ double pe_half(double a) { return 0.5 * a; }
+__device__ __forceinline__ df pe_mul(df a, df b) { return df_mul(a, b); }
+__device__ __forceinline__ df pe_add(df a, df b) { return df_add(a, b); }
+__device__ __forceinline__ df pe_sub(df a, df b) { return df_sub(a, b); }
+__device__ __forceinline__ df pe_neg(df a) { return df_neg(a); }
+__device__ __forceinline__ df pe_half(df a) { return df_scale2(a, 0.5f); }
+__device__ __forceinline__ void pe_const(double x, double& v) { v = x; }
+__device__ __forceinline__ void pe_const(double x, df& v) { v = df_of_f64(x); }
+__device__ __forceinline__ void pe_recip(double c, double& v) { v = 1.0 / c; }
+__device__ __forceinline__ void pe_recip(double c, df& v) { v = df_recip(df_of_f64(c)); }
+// Grid values as stored: in the kernel's arithmetic, or FP64 around a
+// double-float column (split-precision point-set plans).
+template <class V>
+__device__ __forceinline__ V pe_ld(V v) { return v; }
+template <class V, class = std::enable_if_t<std::is_same<V, df>::value>>
+__device__ __forceinline__ df pe_ld(double v) { return df_of_f64(v); }
+__device__ __forceinline__ void pe_st(double& o, double v) { o = v; }
+__device__ __forceinline__ void pe_st(df& o, df v) { o = v; }
+__device__ __forceinline__ void pe_st(double& o, df v) { o = f64_of_df(v); }
+struct PeCol {  // column constants of either arithmetic
+  template <class V>
+  using Sigma = std::conditional_t<std::is_same<V, df>::value, PeSigmaDf, PeSigma>;
+};
+
+constexpr int kPeColWarps = 8;
+
+// One warp per 32 points and every eighth level, the column of each point in
+// shared memory: u, v, T and the running sum are exchanged there, A and G
+// kept for the second pass.  A thread per column (levels in sequence) left
+// 64 x 128 points on a third of the chip and spilled the FP64 column to local
+// memory; the double-float form had to run the first pass twice.
+template <class V, class G>
+__global__ void __launch_bounds__(32 * kPeColWarps) pe_level_columns_kernel(
+    typename PeCol::Sigma<V> sg, long np, int nlon, const double* __restrict__ coslat, const double* __restrict__ fgrid,
+    double f10, long ncolumns, double r_dry, double kappa, const G* grid, G* prod) {
+  extern __shared__ char smem_pe[];
+  V* sh = reinterpret_cast<V*>(smem_pe);  // [6][K][32]: u, v, T, A, G, running sum
+  pdl_wait();
+  const int K = sg.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long col = (long)blockIdx.x * 32 + lane;
+  const bool in = col < ncolumns;
+  const long cc = in ? col : ncolumns - 1;
+  const long b = cc / np, p = cc - b * np;
+  const G* Gd = grid + b * (K + 1) * kPeGrid * np + p;
+  G* P = prod + b * (K + 1) * kPeProd * np + p;
+  V ic, f, kap, rd, zero;
+  pe_recip(coslat[nlon > 0 ? p / nlon : p], ic);
+  pe_const(f10 * fgrid[nlon > 0 ? p / nlon : p], f);
+  pe_const(kappa, kap);
+  pe_const(r_dry, rd);
+  pe_const(0.0, zero);
+  const G* Gs = Gd + (long)K * kPeGrid * np;
+  const V lp_lam = pe_ld<V>(Gs[5 * np]), lp_snt = pe_ld<V>(Gs[6 * np]);
+  auto S = [&](int a, int k) -> V& { return sh[(a * K + k) * 32 + lane]; };
+  for (int k = warp; k < K; k += kPeColWarps) {
+    const G* g = Gd + (long)kPeGrid * k * np;
+    const V u = pe_mul(pe_ld<V>(g[0]), ic), v = pe_mul(pe_ld<V>(g[np]), ic);
+    const V A = pe_mul(pe_sub(pe_mul(u, lp_lam), pe_mul(v, lp_snt)), ic);  // V . grad(ln p_s)
+    const V D = pe_add(pe_ld<V>(g[3 * np]), A);                            // delta + A
+    S(0, k) = u;
+    S(1, k) = v;
+    S(2, k) = pe_ld<V>(g[4 * np]);
+    S(3, k) = A;
+    S(4, k) = D;
+    S(5, k) = pe_mul(sg.dsig[k], D);
+  }
+  __syncthreads();
+  if (warp == 0) {  // cumulative thickness-weighted G, top to bottom
+    V acc = S(5, 0);
+    for (int k = 1; k < K; ++k) {
+      acc = pe_add(acc, S(5, k));
+      S(5, k) = acc;
+    }
+  }
+  __syncthreads();
+  const V total = S(5, K - 1);
+  const V gu = pe_mul(lp_lam, ic), gv = pe_neg(pe_mul(lp_snt, ic));  // grad(ln p_s)
+  if (!in) return;
+  if (warp == K % kPeColWarps) {  // the level of ln p_s
+    G* o = P + (long)K * kPeProd * np;
+    pe_st(o[0], pe_neg(total));  // d ln p_s / dt
+#pragma unroll
+    for (int q = 1; q < kPeProd; ++q) pe_st(o[q * np], zero);
+  }
+  for (int k = warp; k < K; k += kPeColWarps) {
+    const G* g = Gd + (long)kPeGrid * k * np;
+    const V zeta = pe_ld<V>(g[2 * np]), delta = pe_ld<V>(g[3 * np]);
+    const V t_lam = pe_ld<V>(g[5 * np]), t_snt = pe_ld<V>(g[6 * np]);
+    const V e_lam = pe_ld<V>(g[7 * np]), e_snt = pe_ld<V>(g[8 * np]);
+    const V u = S(0, k), v = S(1, k), T = S(2, k), A = S(3, k), D = S(4, k);
+    // interface sigma_dot above and below (exact zeros at the top and the surface)
+    V sd0 = zero, sd1 = zero;
+    if (k > 0) sd0 = pe_sub(pe_mul(sg.s[k], total), S(5, k - 1));
+    if (k + 1 < K) sd1 = pe_sub(pe_mul(sg.s[k + 1], total), S(5, k));
+    auto vadv = [&](int a) {  // centred vertical advection of array a
+      if (K == 1) return zero;
+      V r = zero;
+      if (k + 1 < K) r = pe_mul(sd1, pe_sub(S(a, k + 1), S(a, k)));
+      if (k > 0) {
+        const V up = pe_mul(sd0, pe_sub(S(a, k), S(a, k - 1)));
+        r = k + 1 < K ? pe_add(r, up) : up;
+      }
+      return pe_mul(r, sg.h2[k]);
+    };
+    const V eta = pe_add(zeta, f);
+    V wp = k == 0 ? A : pe_sub(A, pe_mul(sg.bd[k], S(5, k - 1)));
+    wp = pe_sub(wp, pe_mul(sg.alpha[k], D));
+    const V adv_t = pe_mul(pe_sub(pe_mul(u, t_lam), pe_mul(v, t_snt)), ic);
+    G* o = P + (long)kPeProd * k * np;
+    pe_st(o[0], pe_add(pe_sub(pe_neg(adv_t), vadv(2)), pe_mul(pe_mul(kap, T), wp)));
+    pe_st(o[np], pe_neg(pe_add(pe_mul(pe_sub(pe_mul(u, e_lam), pe_mul(v, e_snt)), ic), pe_mul(eta, delta))));
+    pe_st(o[2 * np], pe_add(pe_mul(eta, zeta), pe_mul(pe_add(pe_mul(v, e_lam), pe_mul(u, e_snt)), ic)));
+    pe_st(o[3 * np], pe_half(pe_add(pe_mul(u, u), pe_mul(v, v))));
+    const V rt = pe_mul(rd, T);
+    pe_st(o[4 * np], pe_mul(pe_add(vadv(0), pe_mul(rt, gu)), ic));  // Z / cos
+    pe_st(o[5 * np], pe_mul(pe_add(vadv(1), pe_mul(rt, gv)), ic));
+  }
+}
+
+// What becomes of a tendency value: stored (stage 0) or one RK4 stage update
+// (rk4_stage_kernel's operations and roundings).  ys may be the stage input:
+// each CTA reads what it needs of it before it writes.
+struct PeOut {
+  int stage;
+  double dt;
+  double2 *tend, *y0, *ys, *acc;
+  __device__ __forceinline__ double2 axpy(double2 y, double c, double2 k) const {
+    return make_double2(__dadd_rn(y.x, __dmul_rn(c, k.x)), __dadd_rn(y.y, __dmul_rn(c, k.y)));
+  }
+  __device__ __forceinline__ void put(long i, double2 k) const {
+    if (stage == 0) {
+      tend[i] = k;
+    } else if (stage == 1) {
+      acc[i] = k;
+      ys[i] = axpy(y0[i], 0.5 * dt, k);
+    } else if (stage < 4) {
+      acc[i] = axpy(acc[i], 2.0, k);
+      ys[i] = axpy(y0[i], stage == 2 ? 0.5 * dt : dt, k);
+    } else {
+      const double2 a = acc[i];
+      y0[i] = axpy(y0[i], dt / 6.0, make_double2(__dadd_rn(a.x, k.x), __dadd_rn(a.y, k.y)));
+    }
+  }
+};
+
+// Weak-form curl/div of Z, 2/3 cuts, Simmons-Burridge geopotential of the
+// spectral T (scanned upward in shared memory), -lap(KE + Phi), pins: one
+// warp per 32 (l, m) slots and every eighth level.
+__global__ void __launch_bounds__(32 * kPeColWarps) pe_level_spectral_kernel(PeSigma sg, Spec s, double r_dry, int batch,
+                                                                           const double2* st, const double2* an,
+                                                                           const double2* __restrict__ phis, PeOut out) {
+  extern __shared__ char smem_pe[];
+  double2* below = reinterpret_cast<double2*>(smem_pe);  // [K][32] geopotential under level k, less Phi_s
+  pdl_wait();
+  const int K = sg.K, L = s.L, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long n2 = (long)(L + 1) * (L + 1);
+  const long idx = (long)blockIdx.x * 32 + lane;
+  const bool in = idx < n2 * batch;
+  const long ii = in ? idx : 0;
+  const int b = (int)(ii / n2);
+  const long r = ii - b * n2;
+  const int l = (int)(r / (L + 1)), m = (int)(r - (long)l * (L + 1));
+  const long base = (long)b * (3 * K + 1) * n2 + r;
+  const double2 zero = make_double2(0.0, 0.0);
+  const double2* T = st + base + (long)2 * K * n2;
+  const bool low = in && m <= l;
+  if (low)
+    for (int k = warp; k < K; k += kPeColWarps) below[k * 32 + lane] = T[(long)k * n2];
+  __syncthreads();
+  if (warp == 0 && low) {
+    double2 acc = phis[r];
+    for (int k = K - 1; k >= 0; --k) {
+      const double2 Tk = below[k * 32 + lane];
+      below[k * 32 + lane] = cadd(acc, cscale(r_dry * sg.alpha[k], Tk));  // Phi_k
+      if (k > 0) acc = cadd(acc, cscale(r_dry * sg.beta[k], Tk));
+    }
+  }
+  __syncthreads();
+  if (!in) return;
+  const int cut = (2 * L) / 3;
+  const bool keep = low && l <= cut && m <= cut;
+  const double lap = s.lap(l), mr = (double)m * s.ir;
+  const double cp = keep && l < L ? s.ir * s.cplus[r] : 0.0, cm = keep && l > m ? s.ir * s.cminus[r] : 0.0;
+  for (int k = warp; k <= K; k += kPeColWarps) {
+    const double2* a = an + ((long)b * (K + 1) + k) * kPeProd * n2 + r;
+    if (k == K) {
+      out.put(base + (long)3 * K * n2, keep ? a[0] : zero);
+      continue;
+    }
+    double2 zd = zero, dd = zero, ke = zero, td = zero;
+    if (keep) {
+      const double2 *A = a + 4 * n2, *B = a + 5 * n2;  // analysed Z_east / cos, Z_north / cos
+      auto snt = [&](const double2* c) {               // (1/R) (C+_l c_{l+1} + C-_l c_{l-1})
+        const double2 up = l < L ? c[L + 1] : zero, dn = l > m ? c[-(L + 1)] : zero;
+        return make_double2(fma(cp, up.x, cm * dn.x), fma(cp, up.y, cm * dn.y));
+      };
+      const double2 sa = snt(A), sb = snt(B), al = A[0], bl = B[0];
+      const double2 div = make_double2(fma(-mr, al.y, sb.x), fma(mr, al.x, sb.y));
+      const double2 curl = make_double2(fma(-mr, bl.y, -sa.x), fma(mr, bl.x, -sa.y));
+      td = a[0];
+      zd = csub(a[n2], curl);
+      dd = csub(a[2 * n2], div);
+      ke = a[3 * n2];
+    }
+    out.put(base + (long)(2 * K + k) * n2, td);
+    out.put(base + (long)k * n2, l == 0 ? zero : zd);
+    const double2 phi = low ? below[k * 32 + lane] : zero;
+    out.put(base + (long)(K + k) * n2, l == 0 || !low ? zero : csub(dd, cscale(lap, cadd(ke, phi))));
+  }
+}
+
+size_t pe_grid_bytes(const aeolus_plan_impl* p, int nlev, int batch) {
+  return align256((size_t)batch * (nlev + 1) * kPeGrid * p->npoints * 8);
+}
+size_t pe_prod_bytes(const aeolus_plan_impl* p, int nlev, int batch) {
+  return align256((size_t)batch * (nlev + 1) * kPeProd * p->npoints * 8);
+}
+size_t pe_state_bytes(const aeolus_plan_impl* p, int nlev, int batch) {
+  return align256((size_t)batch * (3 * nlev + 1) * (p->lmax + 1) * (p->lmax + 1) * sizeof(double2));
+}
+size_t pe_bytes(const aeolus_plan_impl* p, int nlev, int batch) {
+  const int bk = batch * (nlev + 1);
+  return pe_grid_bytes(p, nlev, batch) + pe_prod_bytes(p, nlev, batch) +
+         align256((size_t)bk * kPeProd * (p->lmax + 1) * (p->lmax + 1) * sizeof(double2)) +
+         std::max(synth_chain_bytes<kPeGrid, kPeGrid>(p, bk), anal_chain_bytes<kPeProd, kPeProd>(p, bk));
+}
+
+template <class V, class G>
+int launch_pe_columns(const aeolus_plan_impl* p, const typename PeCol::Sigma<V>& sg, double f10, int batch, double r_dry,
+                      double kappa, const void* grid, void* prod, cudaStream_t st) {
+  auto kern = pe_level_columns_kernel<V, G>;
+  const size_t sm = (size_t)6 * sg.K * 32 * sizeof(V);
+  if (int s = allow_smem(kern, sm)) return s;
+  const long ncol = p->npoints * (long)batch;
+  ProfScope prof("pe_columns", st);
+  launch_pdl(kern, dim3(blocks_for(ncol, 32)), dim3(32 * kPeColWarps), sm, st, sg, p->npoints,
+             p->kind == kGauss ? p->nlon : 0, static_cast<const double*>(p->coslat),
+             static_cast<const double*>(p->fgrid), f10, ncol, r_dry, kappa, static_cast<const G*>(grid),
+             static_cast<G*>(prod));
+  AE_LAUNCH("pe_level_columns_kernel");
+  return AEOLUS_OK;
+}
+
+int pe_chain(const aeolus_plan_impl* p, const aeolus_pe_params* prm, const PeSigma& sg, const double2* state,
+             const double2* phi_s, const PeOut& out, int batch, void* work, cudaStream_t st) {
+  const int K = sg.K, bk = batch * (K + 1);
+  const long np = p->npoints;
+  char* w = static_cast<char*>(work);
+  double* grid = reinterpret_cast<double*>(w);
+  w += pe_grid_bytes(p, K, batch);
+  double* prod = reinterpret_cast<double*>(w);
+  w += pe_prod_bytes(p, K, batch);
+  double2* an = reinterpret_cast<double2*>(w);
+  w += align256((size_t)bk * kPeProd * (p->lmax + 1) * (p->lmax + 1) * sizeof(double2));
+  const Spec sp = make_spec(p, prm->radius);
+  const double f10 = 2.0 * prm->omega * kSqrt4PiOver3, kappa = prm->r_dry / prm->cp_dry;
+  const PeDerive d{sp, state, K, f10};
+  const PeEpi e{an, p->lmax};
+  int s;
+  if (split_on(p)) {
+    if ((s = run_synth_chain<PeDerive, PePw, kOutGridDf>(p, d, PePw{}, bk, grid, kPeGrid * np, np, w, nullptr, st)) ||
+        (s = launch_pe_columns<df, df>(p, sigma_df(sg), f10, batch, prm->r_dry, kappa, grid, prod, st)) ||
+        (s = run_anal_chain<PwCopyN<kPeProd>, PeEpi, kInGridDf>(p, PwCopyN<kPeProd>{}, e, bk, prod, kPeProd * np, np, w,
+                                                                st)))
+      return s;
+  } else {
+    if ((s = run_synth_chain(p, d, PePw{}, bk, grid, kPeGrid * np, np, w, nullptr, st)) ||
+        (s = p->precision == AEOLUS_PREC_SPLIT_BF16
+                 ? launch_pe_columns<df, double>(p, sigma_df(sg), f10, batch, prm->r_dry, kappa, grid, prod, st)
+                 : launch_pe_columns<double, double>(p, sg, f10, batch, prm->r_dry, kappa, grid, prod, st)) ||
+        (s = run_anal_chain(p, PwCopyN<kPeProd>{}, e, bk, prod, kPeProd * np, np, w, st)))
+      return s;
+  }
+  const size_t sm = (size_t)K * 32 * sizeof(double2);
+  const long n = (long)(p->lmax + 1) * (p->lmax + 1) * batch;
+  ProfScope prof("pe_spectral", st);
+  launch_pdl(pe_level_spectral_kernel, dim3(blocks_for(n, 32)), dim3(32 * kPeColWarps), sm, st, sg, sp, prm->r_dry, batch,
+             state, static_cast<const double2*>(an), phi_s, out);
+  AE_LAUNCH("pe_level_spectral_kernel");
+  return AEOLUS_OK;
+}
+
+int pe_chain_check(aeolus_plan plan, const aeolus_pe_params* prm, int nlev, const double* interfaces, const void* state,
+                   const void* phi_s, const void* out, int batch, const char* who, PeSigma* sg) {
+  if (int s = check_common(plan, who, batch, state, out)) return s;
+  if (int s = pe_check(prm)) return s;
+  if (int s = make_sigma(interfaces, nlev, sg)) return s;
+  if (batch > 0 && !phi_s) return fail(AEOLUS_ERR_ARG, std::string(who) + ": NULL phi_s");
+  if ((long)batch * (nlev + 1) > 65535)
+    return fail(AEOLUS_ERR_ARG, std::string(who) + ": batch (nlev + 1) above 65535");
+  return AEOLUS_OK;
+}
+
 // One classical RK4 stage update over n complex values, in the reference's
 // order of operations (run/engine.py:406-431), with every FP64 product and
 // sum rounded separately (no contraction into FMAs), as NumPy/torch do:
@@ -567,5 +1058,52 @@ extern "C" int aeolus_pe_spectral(int lmax, const aeolus_pe_params* prm, int nle
       reinterpret_cast<const double2*>(div_z), reinterpret_cast<const double2*>(phi_s),
       reinterpret_cast<double2*>(tendency));
   AE_LAUNCH("pe_spectral_kernel");
+  return AEOLUS_OK;
+}
+
+extern "C" int aeolus_pe_workspace_bytes(aeolus_plan plan, int nlev, int batch, size_t* tendency_bytes,
+                                         size_t* rk4_bytes) {
+  if (!plan_ok(plan) || nlev < 1 || nlev > kPeMaxLevels || batch < 0)
+    return fail(AEOLUS_ERR_ARG, "aeolus_pe_workspace_bytes: bad arguments");
+  const size_t n = pe_bytes(plan, nlev, std::max(batch, 1));
+  if (tendency_bytes) *tendency_bytes = n;
+  if (rk4_bytes) *rk4_bytes = n + 2 * pe_state_bytes(plan, nlev, std::max(batch, 1));
+  return AEOLUS_OK;
+}
+
+extern "C" int aeolus_pe_tendency(aeolus_plan plan, const aeolus_pe_params* prm, int nlev, const double* interfaces,
+                                  const double* state, const double* phi_s, double* tendency, int batch, void* work,
+                                  size_t work_bytes, void* stream) {
+  PeSigma sg;
+  if (int s = pe_chain_check(plan, prm, nlev, interfaces, state, phi_s, tendency, batch, "aeolus_pe_tendency", &sg))
+    return s;
+  if (batch == 0) return AEOLUS_OK;
+  if (!work || work_bytes < pe_bytes(plan, nlev, batch))
+    return fail(AEOLUS_ERR_WORKSPACE, "aeolus_pe_tendency: workspace too small");
+  const PeOut out{0, 0.0, reinterpret_cast<double2*>(tendency), nullptr, nullptr, nullptr};
+  return pe_chain(plan, prm, sg, reinterpret_cast<const double2*>(state), reinterpret_cast<const double2*>(phi_s), out,
+                  batch, work, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int aeolus_pe_rk4(aeolus_plan plan, const aeolus_pe_params* prm, int nlev, const double* interfaces,
+                             double* state, const double* phi_s, int batch, double dt, int nsteps, void* work,
+                             size_t work_bytes, void* stream) {
+  PeSigma sg;
+  if (int s = pe_chain_check(plan, prm, nlev, interfaces, state, phi_s, state, batch, "aeolus_pe_rk4", &sg)) return s;
+  if (!std::isfinite(dt)) return fail(AEOLUS_ERR_ARG, "aeolus_pe_rk4: dt must be finite");
+  if (batch == 0 || nsteps <= 0) return AEOLUS_OK;
+  const size_t nb = pe_bytes(plan, nlev, batch), ns = pe_state_bytes(plan, nlev, batch);
+  if (!work || work_bytes < nb + 2 * ns) return fail(AEOLUS_ERR_WORKSPACE, "aeolus_pe_rk4: workspace too small");
+  char* w = static_cast<char*>(work);
+  double2* y0 = reinterpret_cast<double2*>(state);
+  double2* ys = reinterpret_cast<double2*>(w + nb);
+  double2* acc = reinterpret_cast<double2*>(w + nb + ns);
+  for (int it = 0; it < nsteps; ++it)
+    for (int stage = 1; stage <= 4; ++stage) {
+      const PeOut out{stage, dt, nullptr, y0, ys, acc};
+      if (int s = pe_chain(plan, prm, sg, stage == 1 ? y0 : ys, reinterpret_cast<const double2*>(phi_s), out, batch,
+                           work, static_cast<cudaStream_t>(stream)))
+        return s;
+    }
   return AEOLUS_OK;
 }

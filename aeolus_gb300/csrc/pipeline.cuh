@@ -266,19 +266,23 @@ int launch_rows(const aeolus_plan_impl* p, const Pw& pw, RowArgs a, cudaStream_t
       default: return launch_rows_fx<Pw, IN_MODE, OUT_MODE, FftRuntime>(p, pw, a, st);
     }
   }
-  const WideRowCfg c = wide_row_cfg<Pw>(p, a.batch);
-  const char* name = IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_c2r_products_r2c" : "rows_c2r") : "rows_r2c";
-  constexpr int NR = w_rows_per_cta<Pw>();
-  auto kern = c.nr == 1 ? row_kernel_w<Pw, 1, IN_MODE, OUT_MODE> : row_kernel_w<Pw, NR, IN_MODE, OUT_MODE>;
-  auto kdft = c.gtab ? row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, true> : row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, false>;
-  int s = p->fftx.use_fft ? allow_smem(kern, c.smem) : allow_smem(kdft, c.smem);
-  if (s) return s;
-  ProfScope prof(name, st);
-  const FxW* tw = p->twfx;
-  if (p->fftx.use_fft) launch_pdl(kern, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, fx_consts());
-  else launch_pdl(kdft, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, c.gf);
-  AE_LAUNCH("row_kernel_w");
-  return AEOLUS_OK;
+  if constexpr (IN_MODE == kInGridDf || OUT_MODE == kOutGridDf) {
+    return fail(AEOLUS_ERR_ARG, "double-float grids need a split-precision Gauss plan");
+  } else {
+    const WideRowCfg c = wide_row_cfg<Pw>(p, a.batch);
+    const char* name = IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_c2r_products_r2c" : "rows_c2r") : "rows_r2c";
+    constexpr int NR = w_rows_per_cta<Pw>();
+    auto kern = c.nr == 1 ? row_kernel_w<Pw, 1, IN_MODE, OUT_MODE> : row_kernel_w<Pw, NR, IN_MODE, OUT_MODE>;
+    auto kdft = c.gtab ? row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, true> : row_kernel_w_dft<Pw, IN_MODE, OUT_MODE, false>;
+    int s = p->fftx.use_fft ? allow_smem(kern, c.smem) : allow_smem(kdft, c.smem);
+    if (s) return s;
+    ProfScope prof(name, st);
+    const FxW* tw = p->twfx;
+    if (p->fftx.use_fft) launch_pdl(kern, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, fx_consts());
+    else launch_pdl(kdft, c.grid, dim3(c.threads), c.smem, st, a, pw, tw, c.gf);
+    AE_LAUNCH("row_kernel_w");
+    return AEOLUS_OK;
+  }
 }
 
 // Bytes of the F/G block area for `nblk` fields per (member, row).

@@ -7,8 +7,11 @@
 
 namespace aeolus {
 
-enum { kInF = 0, kInGrid = 1 };
-enum { kOutGrid = 0, kOutG = 1 };
+// Row inputs and outputs: order spectra, an FP64 grid, or (split-precision
+// plans) a grid of double-floats, which saves the conversions on both sides
+// of a double-float kernel.
+enum { kInF = 0, kInGrid = 1, kInGridDf = 2 };
+enum { kOutGrid = 0, kOutG = 1, kOutGridDf = 2 };
 
 struct RowArgs {
   int L, nlat, batch;
@@ -30,6 +33,15 @@ struct RowArgs {
   // kOutGrid: out[b * gout_b + f * gout_f + j * N + k]
   double* gout;
   long gout_b, gout_f;
+  template <int MODE>
+  __device__ __forceinline__ df in_df(long i) const {  // grid value i as a double-float
+    return MODE == kInGridDf ? reinterpret_cast<const df*>(gin)[i] : df_of_f64(gin[i]);
+  }
+  template <int MODE>
+  __device__ __forceinline__ void put_df(long i, df v) const {
+    if (MODE == kOutGridDf) reinterpret_cast<df*>(gout)[i] = v;
+    else gout[i] = f64_of_df(v);
+  }
   unsigned* status;       // optional per-member state bits
   double ir;              // 1 / R of the functor's longitude derivatives (RowSrc)
   int drop;               // kOutG: orders above L - drop are not written (EpiTop)

@@ -418,7 +418,7 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
     df* x0 = reinterpret_cast<df*>(buf0);
     for (int idx = threadIdx.x; idx < NIN * N; idx += blockDim.x) {
       const int f = idx / N, k = idx - f * N;
-      x0[(long)f * 2 * ns + k] = df_of_f64(a.gin[(long)b * a.gin_b + (long)f * a.gin_f + (long)j * N + k]);
+      x0[(long)f * 2 * ns + k] = a.in_df<IN_MODE>((long)b * a.gin_b + (long)f * a.gin_f + (long)j * N + k);
     }
     __syncthreads();
   }
@@ -464,10 +464,10 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
   if (a.status && threadIdx.x == 0 && s_bits) atomicOr(&a.status[b], s_bits);
 
   // ---- 3. outputs
-  if (OUT_MODE == kOutGrid) {
+  if (OUT_MODE != kOutG) {
     for (int idx = threadIdx.x; idx < NOUT * N; idx += blockDim.x) {
       const int f = idx / N, k = idx - f * N;
-      a.gout[(long)b * a.gout_b + (long)f * a.gout_f + (long)j * N + k] = f64_of_df(xout[(long)f * 2 * ns + k]);
+      a.put_df<OUT_MODE>((long)b * a.gout_b + (long)f * a.gout_f + (long)j * N + k, xout[(long)f * 2 * ns + k]);
     }
   } else if (use_fft) {
     // output block exponents (|X| < 2^hb)
@@ -703,7 +703,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
     for (int idx = tid; idx < NIN * N; idx += T) {
       const int f = idx / N, k = idx - f * N;
       x0[2 * (f * fs + Row::swz(k >> 1)) + (k & 1)] =
-          df_of_f64(a.gin[(long)b * a.gin_b + (long)f * a.gin_f + (long)j * N + k]);
+          a.in_df<IN_MODE>((long)b * a.gin_b + (long)f * a.gin_f + (long)j * N + k);
     }
     __syncthreads();
   }
@@ -758,11 +758,11 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
   if (a.status && tid == 0 && s_bits) atomicOr(&a.status[b], s_bits);
 
   // ---- 3. outputs
-  if constexpr (OUT_MODE == kOutGrid) {
+  if constexpr (OUT_MODE != kOutG) {
     for (int idx = tid; idx < NOUT * N; idx += T) {
       const int f = idx / N, k = idx - f * N;
-      a.gout[(long)b * a.gout_b + (long)f * a.gout_f + (long)j * N + k] =
-          f64_of_df(xout[2 * (f * fs + Row::swz(k >> 1)) + (k & 1)]);
+      a.put_df<OUT_MODE>((long)b * a.gout_b + (long)f * a.gout_f + (long)j * N + k,
+                         xout[2 * (f * fs + Row::swz(k >> 1)) + (k & 1)]);
     }
   } else {
     if (tid < NOUT) {

@@ -357,7 +357,7 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
       const int rf = idx / N, k = idx - rf * N, row = rf / NIN, f = rf - row * NIN;
       if (row < nrow)
         reinterpret_cast<df*>(zrow(row, f))[2 * s_grid[k >> 1] + (k & 1)] =
-            df_of_f64(a.gin[(long)(b0 + row) * a.gin_b + (long)f * a.gin_f + (long)j * N + k]);
+            a.in_df<IN_MODE>((long)(b0 + row) * a.gin_b + (long)f * a.gin_f + (long)j * N + k);
     }
     __syncthreads();
   }
@@ -467,13 +467,13 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
   if (a.status && tid < nrow && s_bits[tid]) atomicOr(&a.status[b0 + tid], s_bits[tid]);
 
   // ---- 3. outputs
-  if constexpr (OUT_MODE == kOutGrid) {
+  if constexpr (OUT_MODE != kOutG) {
 #pragma unroll 1
     for (int idx = tid; idx < NRO * N; idx += T) {
       const int rf = idx / N, k = idx - rf * N, row = rf / NOUT, f = rf - row * NOUT;
       if (row < nrow)
-        a.gout[(long)(b0 + row) * a.gout_b + (long)f * a.gout_f + (long)j * N + k] =
-            f64_of_df(reinterpret_cast<const df*>(zrow(row, f))[2 * s_grid[k >> 1] + (k & 1)]);
+        a.put_df<OUT_MODE>((long)(b0 + row) * a.gout_b + (long)f * a.gout_f + (long)j * N + k,
+                           reinterpret_cast<const df*>(zrow(row, f))[2 * s_grid[k >> 1] + (k & 1)]);
     }
   } else {
     if (tid < NRO) {  // output block exponents (|X| < 2^hb)

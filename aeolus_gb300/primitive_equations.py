@@ -3,19 +3,16 @@
 Mirrors src/planetary_sandbox/physics/sigma_coordinate.py:38-149 (the
 Lorenz sigma grid) and physics/primitive_equations.py:40-753 (state layout,
 isothermal rest state, model constructor checks and the explicit tendency).
-The tendency runs on the device, batched over levels and members:
-
-  aeolus_pe_derive    spectral derivative fields of every level
-  aeolus_synthesize   10 K + 2 fields per member on the product plan
-  aeolus_pe_columns   the vertical column physics at every product point
-  aeolus_analyze      4 K + 1 integrands per member
-  aeolus_vector_curl_div  weak-form curl/div of Z on the extended plan
-  aeolus_pe_spectral  2/3 cuts, Simmons-Burridge geopotential, l = 0 pins
+The tendency is one library call (``aeolus_pe_tendency``), batched over
+levels and members on the product plan: synthesis of every level's fields, the
+vertical column physics at every product point, analysis of the integrands,
+then the weak-form curl/div, 2/3 cuts, Simmons-Burridge geopotential and l = 0
+pins; ``aeolus_pe_rk4`` runs whole steps of it.
 """
 from __future__ import annotations
 
 import math
-from ctypes import byref, c_void_p
+from ctypes import byref, c_size_t, c_void_p
 from dataclasses import dataclass
 from functools import cached_property
 
@@ -24,7 +21,7 @@ import torch
 
 from . import _lib
 from ._lib import check
-from .ops import analyze, spectral_op, synthesize, vector_curl_div, winds
+from .ops import _stream, spectral_op, synthesize, winds
 
 R_DRY = 287.04          # J kg^-1 K^-1, primitive_equations.py:49
 CP_DRY = 1004.64        # J kg^-1 K^-1
@@ -196,6 +193,13 @@ class PrimitiveEquationsModel:
     def _ext_plan(self):
         return self.so._extended_plan()
 
+    def _workspace(self, batch: int, rk4: int, device) -> torch.Tensor:
+        """Scratch of one tendency (rk4 = 0) or of RK4 steps (rk4 = 1)."""
+        nb = (c_size_t(), c_size_t())
+        check(_lib.load().aeolus_pe_workspace_bytes(self._plan.handle, self.nlev, int(batch), byref(nb[0]),
+                                                    byref(nb[1])))
+        return torch.empty(nb[rk4].value, dtype=torch.uint8, device=device)
+
     def tendency(self, coeffs: torch.Tensor) -> torch.Tensor:
         """d/dt of the (..., 3K+1, L+1, L+1) stack (:727-753)."""
         K, L = self.nlev, self.l_max
@@ -212,25 +216,10 @@ class PrimitiveEquationsModel:
         out = torch.empty_like(x)
         if B == 0:
             return out.reshape(lead + (3 * K + 1, n, n))
-        lib = _lib.load()
-        dev = x.device
-        stream = c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        plan = self._plan
-        fields = torch.empty((B, 10 * K + 2, n, n), dtype=torch.complex128, device=dev)
-        check(lib.aeolus_pe_derive(plan.handle, byref(self._params), K, _p(x), _p(fields), B, stream))
-        grid = synthesize(plan.id, fields)                                  # [B, 10K+2, np]
-        npts = grid.shape[-1]
-        prod = torch.empty((B, 4 * K + 1, npts), dtype=torch.float64, device=dev)
-        fen = torch.empty((B * K, 2, npts), dtype=torch.float64, device=dev)
-        sig = self._sigma_host
-        check(lib.aeolus_pe_columns(plan.handle, byref(self._params), K, sig.ctypes.data_as(c_void_p), _p(grid),
-                                    _p(prod), _p(fen), B, stream))
-        an = analyze(plan.id, prod)                                         # [B, 4K+1, n, n]
-        ext = self._ext_plan()
-        cd = vector_curl_div(ext.id, self.R, fen[:, 0], fen[:, 1], False)   # [2, B*K, n, n]
-        curl_z, div_z = cd[0].contiguous(), cd[1].contiguous()
-        check(lib.aeolus_pe_spectral(L, byref(self._params), K, sig.ctypes.data_as(c_void_p), _p(x), _p(an),
-                                     _p(curl_z), _p(div_z), _p(self.phi_surface_lm), _p(out), B, stream))
+        work = self._workspace(B, 0, x.device)
+        check(_lib.load().aeolus_pe_tendency(self._plan.handle, byref(self._params), K,
+                                             self._sigma_host.ctypes.data_as(c_void_p), _p(x), _p(self.phi_surface_lm),
+                                             _p(out), B, _p(work), work.numel(), _stream(x.device)))
         return out.reshape(lead + (3 * K + 1, n, n))
 
     def tendency_state(self, state: PrimitiveEquationsState) -> PrimitiveEquationsState:
@@ -244,6 +233,19 @@ class PrimitiveEquationsModel:
         from .engine import rk4_step_device
 
         y = torch.as_tensor(coeffs).to(torch.complex128).contiguous()
+        K, n = self.nlev, self.l_max + 1
+        if stage_validator is None and y.is_cuda and tuple(y.shape[-3:]) == (3 * K + 1, n, n) and y.numel():
+            # all stages in one library call: the generic step's operations
+            # and roundings on the same tendencies
+            y = y.clone()
+            B = y.numel() // ((3 * K + 1) * n * n)
+            if nsteps > 0:
+                work = self._workspace(B, 1, y.device)
+                check(_lib.load().aeolus_pe_rk4(self._plan.handle, byref(self._params), K,
+                                                self._sigma_host.ctypes.data_as(c_void_p), _p(y),
+                                                _p(self.phi_surface_lm), B, float(dt), int(nsteps), _p(work),
+                                                work.numel(), _stream(y.device)))
+            return y
         for _ in range(int(nsteps)):
             y = rk4_step_device(self.tendency, y, 0.0, dt, stage_validator=stage_validator)
         return y

@@ -261,6 +261,21 @@ int aeolus_pe_spectral(int lmax, const aeolus_pe_params* params, int nlev, const
                        const double* state, const double* analysed, const double* curl_z, const double* div_z,
                        const double* phi_s, double* tendency, int batch, void* stream);
 
+/* The whole tendency (and RK4 steps) of primitive_equations.py:727-753 on
+ * the device: the same maths as the calls above as one chain of fused kernels
+ * on the product plan (any plan kind and precision; no extended plan, since
+ * the 2/3 cut keeps curl/div degrees below l_max).  state [batch][3K+1][L+1]
+ * [L+1], phi_s [L+1][L+1], device; `interfaces` host.  aeolus_pe_rk4 advances
+ * `state` in place by nsteps classical steps, the operations and roundings of
+ * aeolus_rk4_stage on these tendencies.  Workspace sizes (either pointer may
+ * be NULL) from aeolus_pe_workspace_bytes; batch (K + 1) is at most 65535. */
+int aeolus_pe_workspace_bytes(aeolus_plan plan, int nlev, int batch, size_t* tendency_bytes, size_t* rk4_bytes);
+int aeolus_pe_tendency(aeolus_plan plan, const aeolus_pe_params* params, int nlev, const double* interfaces,
+                       const double* state, const double* phi_s, double* tendency, int batch, void* work,
+                       size_t work_bytes, void* stream);
+int aeolus_pe_rk4(aeolus_plan plan, const aeolus_pe_params* params, int nlev, const double* interfaces, double* state,
+                  const double* phi_s, int batch, double dt, int nsteps, void* work, size_t work_bytes, void* stream);
+
 /* One classical RK4 stage update of n complex values (y0, k, ystage, acc
  * are [n] complex128 device arrays), the device form of the reference's
  * rk4_step_array (run/engine.py:406-431) for any tendency (the primitive
