@@ -42,6 +42,26 @@ struct RowArgs {
     if (MODE == kOutGridDf) reinterpret_cast<df*>(gout)[i] = v;
     else gout[i] = f64_of_df(v);
   }
+  // grid values i (even) and i + 1 on the packed lanes
+  template <int MODE>
+  __device__ __forceinline__ df2 in_df2(long i) const {
+    if (MODE == kInGridDf) {
+      const float4 w = *reinterpret_cast<const float4*>(reinterpret_cast<const df*>(gin) + i);
+      return df2{f2_pack(w.x, w.z), f2_pack(w.y, w.w)};
+    }
+    return df2_pack(df_of_f64(gin[i]), df_of_f64(gin[i + 1]));
+  }
+  template <int MODE>
+  __device__ __forceinline__ void put_df2(long i, df2 v) const {
+    df a, b;
+    df2_unpack(v, a, b);
+    if (MODE == kOutGridDf) {
+      *reinterpret_cast<float4*>(reinterpret_cast<df*>(gout) + i) = make_float4(a.hi, a.lo, b.hi, b.lo);
+    } else {
+      gout[i] = f64_of_df(a);
+      gout[i + 1] = f64_of_df(b);
+    }
+  }
   unsigned* status;       // optional per-member state bits
   double ir;              // 1 / R of the functor's longitude derivatives (RowSrc)
   int drop;               // kOutG: orders above L - drop are not written (EpiTop)
