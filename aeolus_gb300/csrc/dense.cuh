@@ -47,8 +47,11 @@ inline DenseDims dense_dims(int M, int N, int K, int sm_count) {
   return d;
 }
 
-// Units (M tile, N tile, K part), K part slowest so neighbouring CTAs share
-// data tiles.
+// Units (K part, M tile, N tile), N tile fastest: the CTAs that contract the
+// same basis rows with different data columns run side by side, so the basis
+// digits (12 bytes per entry, far more than L2 holds) come from HBM once per
+// product and not once per 32 data columns: 64 fields at level 6, l_max 127
+// (8.05 GB of digits) 2.28 -> 1.66 ms per product.
 struct DenseSched {
   static constexpr int kSegChunks = kDenseSegChunks;
   DenseDims d;
@@ -58,7 +61,7 @@ struct DenseSched {
   int count_host() const { return count(); }
   __device__ TcTile tile(int t) const {
     const int kp = t / (d.Mt * d.Nt), r = t - kp * d.Mt * d.Nt;
-    const int nt = r / d.Mt, mt = r - nt * d.Mt;
+    const int mt = r / d.Nt, nt = r - mt * d.Nt;
     const int k0 = kp * d.cpp, k1 = min(d.nkc, k0 + d.cpp);
     return TcTile{A + ((long long)mt * d.nkc + k0) * chunk_elems(128),
                   B + ((long long)nt * d.nkc + k0) * chunk_elems(kNT), k1 - k0};
@@ -106,7 +109,7 @@ struct DenseEpi {
   }
   __device__ void seg_end(int t, const State& st, int row, int c0, int) const {
     const int kp = t / (d.Mt * d.Nt), r = t - kp * d.Mt * d.Nt;
-    const int nt = r / d.Mt, mt = r - nt * d.Mt;
+    const int mt = r / d.Nt, nt = r - mt * d.Nt;
     const int m = mt * 128 + row;
     const int ea = eA[m];
     const long long ldp = (long long)d.Mt * 128;
