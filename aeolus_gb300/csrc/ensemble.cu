@@ -61,6 +61,7 @@ template <class Derive>
 struct SynthArg {
   LegArgs a;
   Derive d;
+  int cpt;  // columns per thread
 };
 template <class Epi>
 struct AnalArg {
@@ -101,7 +102,8 @@ __global__ void __launch_bounds__(256) g_legendre_synth(Grouped<SynthArg<Derive>
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
-  legendre_synth_body<Derive>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
+  if (g.arg[k].cpt == 2) legendre_synth_body<Derive, 2>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
+  else legendre_synth_body<Derive, 1>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
 }
 
 template <class Epi>
@@ -394,10 +396,10 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
       double2* FG = reinterpret_cast<double2*>(chain[k]);
       const LegCfg cs = synth_cfg<SDerive>(p, E->batch[k]);
       const LegCfg ca = analysis_cfg<Epi>(p, E->batch[k]);
-      grouped_add(gs, SynthArg<SDerive>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], cs.bc, cs.ss, p->P, p->PT, FG, N64},
-                                        M::split_derive(der[k])},
+      grouped_add(gs, SynthArg<SDerive>{leg_args(p, cs, E->batch[k], FG, N64),
+                                        M::split_derive(der[k]), cs.cpt},
                   cs.grid);
-      grouped_add(ga, AnalArg<Epi>{LegArgs{p->lmax, p->nlat, p->nh, E->batch[k], ca.bc, ca.ss, p->P, p->PT, FG, N64}, epi[k]},
+      grouped_add(ga, AnalArg<Epi>{leg_args(p, ca, E->batch[k], FG, N64), epi[k]},
                   ca.grid);
       sm_s = std::max(sm_s, cs.smem);
       sm_a = std::max(sm_a, ca.smem);

@@ -35,137 +35,10 @@
 // 3.34e-15, delta 9.04e-13 -> 9.01e-13, phi 1.95e-15 -> 1.93e-15.
 #pragma once
 
-#include "fx.cuh"
 #include "rows.cuh"
+#include "w96.cuh"
 
 namespace aeolus {
-
-// ------------------------------------------------------- 96-bit integers
-struct w96 {
-  unsigned l, m;
-  int h;
-};
-struct cw {
-  w96 re, im;
-};
-
-__device__ __forceinline__ w96 w_add(w96 a, w96 b) {
-  w96 r;
-  asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
-      : "=r"(r.l), "=r"(r.m), "=r"(r.h)
-      : "r"(a.l), "r"(a.m), "r"(a.h), "r"(b.l), "r"(b.m), "r"(b.h));
-  return r;
-}
-__device__ __forceinline__ w96 w_sub(w96 a, w96 b) {
-  w96 r;
-  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
-      : "=r"(r.l), "=r"(r.m), "=r"(r.h)
-      : "r"(a.l), "r"(a.m), "r"(a.h), "r"(b.l), "r"(b.m), "r"(b.h));
-  return r;
-}
-__device__ __forceinline__ w96 w_neg(w96 a) { return w_sub(w96{0u, 0u, 0}, a); }
-__device__ __forceinline__ w96 w_half(w96 a) {
-  return w96{__funnelshift_r(a.l, a.m, 1), __funnelshift_r(a.m, (unsigned)a.h, 1), a.h >> 1};
-}
-// v 2^s for a 64-bit v, 0 <= s < 32.
-__device__ __forceinline__ w96 w_shl64(long long v, int s) {
-  const unsigned lo = (unsigned)v, hi = (unsigned)((unsigned long long)v >> 32);
-  return w96{lo << s, __funnelshift_l(lo, hi, s), (int)__funnelshift_l(hi, (unsigned)((int)hi >> 31), s)};
-}
-
-// 30-bit limbs x = x2 2^60 + (X1 / 2) 2^30 + X0 / 2 (|x| < 2^90): the two low
-// ones doubled, to pair with the 31-bit limbs of a Q61 factor.
-struct wlimbs {
-  int x2, x1, X1, X0;
-};
-__device__ __forceinline__ wlimbs w_limbs(w96 x) {
-  const int X1 = (int)(__funnelshift_r(x.l, x.m, 29) & 0x7FFFFFFEu);
-  return wlimbs{(int)__funnelshift_r(x.m, (unsigned)x.h, 28), X1 >> 1, X1, (int)((x.l << 1) & 0x7FFFFFFEu)};
-}
-// (H 2^31 + T2) / 2 with H = sum of x2 wh, T2 = sum of x2 wl + X1 wh + carry.
-__device__ __forceinline__ w96 w_recombine(long long H, long long T2) {
-  const unsigned hl = (unsigned)H, hh = (unsigned)((unsigned long long)H >> 32);
-  const unsigned tl = (unsigned)T2, th = (unsigned)((unsigned long long)T2 >> 32);
-  return w_add(w96{hl << 30, __funnelshift_r(hl, hh, 2), (int)hh >> 2},
-               w96{__funnelshift_r(tl, th, 1), (unsigned)((int)th >> 1), (int)th >> 31});
-}
-// x k, |k| <= 1.
-__device__ __forceinline__ w96 w_mulk(w96 x, FxK k) {
-  const wlimbs a = w_limbs(x);
-  const long long t1 = fx_madw(a.X0, k.h, fx_madw(a.x1, k.l, 0LL));
-  const long long t2 = fx_madw(a.X1, k.h, fx_madw(a.x2, k.l, t1 >> 30));
-  return w_recombine(fx_madw(a.x2, k.h, 0LL), t2);
-}
-// x w (CONJ: x conj(w)), |w| = 1.
-template <bool CONJ>
-__device__ __forceinline__ cw w_cmul(cw x, FxW w) {
-  const wlimbs a = w_limbs(x.re), b = w_limbs(x.im);
-  // re = a c -+ b s, im = +-a s + b c: the sign goes to s
-  const int sh = w.sh, sl = w.sl, nh = -w.sh, nl = -w.sl;
-  const int rh = CONJ ? sh : nh, rl = CONJ ? sl : nl;  // factor of b in re
-  const int ih = CONJ ? nh : sh, il = CONJ ? nl : sl;  // factor of a in im
-  const long long r1 = fx_madw(b.X0, rh, fx_madw(b.x1, rl, fx_madw(a.X0, w.ch, fx_madw(a.x1, w.cl, 0LL))));
-  const long long r2 =
-      fx_madw(b.X1, rh, fx_madw(b.x2, rl, fx_madw(a.X1, w.ch, fx_madw(a.x2, w.cl, r1 >> 30))));
-  const long long i1 = fx_madw(b.X0, w.ch, fx_madw(b.x1, w.cl, fx_madw(a.X0, ih, fx_madw(a.x1, il, 0LL))));
-  const long long i2 =
-      fx_madw(b.X1, w.ch, fx_madw(b.x2, w.cl, fx_madw(a.X1, ih, fx_madw(a.x2, il, i1 >> 30))));
-  return cw{w_recombine(fx_madw(b.x2, rh, fx_madw(a.x2, w.ch, 0LL)), r2),
-            w_recombine(fx_madw(b.x2, w.ch, fx_madw(a.x2, ih, 0LL)), i2)};
-}
-__device__ __forceinline__ cw cw_add(cw a, cw b) { return cw{w_add(a.re, b.re), w_add(a.im, b.im)}; }
-__device__ __forceinline__ cw cw_sub(cw a, cw b) { return cw{w_sub(a.re, b.re), w_sub(a.im, b.im)}; }
-// a + sg i b and a - sg i b (sg = +1 for POS) without a negation
-template <bool POS>
-__device__ __forceinline__ cw cw_add_i(cw a, cw b) {
-  return POS ? cw{w_sub(a.re, b.im), w_add(a.im, b.re)} : cw{w_add(a.re, b.im), w_sub(a.im, b.re)};
-}
-
-// ------------------------------------------------- FP64 <-> fixed point
-// Key of |x|: its high word (exponent and 20 mantissa bits).
-__device__ __forceinline__ unsigned f64_key(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
-constexpr unsigned kNonFinite = 0x7FF00000u;  // keys from here on are infinities and NaNs
-// Exponent E with |x| < 2^E for every finite x whose key is at most `key`.
-__device__ __forceinline__ int f64_key_exp(unsigned key) { return max((int)(key >> 20), 1) - 1022; }
-
-// x 2^-S towards zero, for |x 2^-S| < 2^84.
-__device__ __forceinline__ w96 w_of_f64(double x, int S) {
-  const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
-  const int ex = (int)((xh >> 20) & 0x7FFu);
-  const unsigned mh = (xh & 0xFFFFFu) | (ex ? 0x100000u : 0u);
-  // mantissa left-aligned in 96 bits (2^43 times its value), then shifted down
-  unsigned h = __funnelshift_l(xl, mh, 11), m = xl << 11, l = 0u;
-  int r = 1118 + S - max(ex, 1);  // 43 - (ex - 1075 - S)
-  if (r >= 64) l = h, m = 0u, h = 0u, r -= 64;
-  else if (r >= 32) l = m, m = h, h = 0u, r -= 32;
-  if (r >= 32) l = 0u, r = 0;  // below one unit
-  l = __funnelshift_r(l, m, r);
-  m = __funnelshift_r(m, h, r);
-  h = h >> r;
-  const w96 v{l, m, (int)h};
-  return (int)xh < 0 ? w_neg(v) : v;
-}
-
-// X 2^S rounded to FP64 (half up in magnitude; results below the normal range
-// are zero, above it infinite), integer instructions only.
-__device__ __forceinline__ double f64_of_w(w96 x, int S) {
-  const int s = x.h >> 31;
-  unsigned h = (unsigned)(x.h ^ s), m = x.m ^ (unsigned)s, l = x.l ^ (unsigned)s;  // |x| (one unit less if negative)
-  int top = 95;
-  if (h == 0u) h = m, m = l, l = 0u, top = 63;
-  if (h == 0u) h = m, m = 0u, top -= 32;
-  const int c = __clz((int)h);
-  if (c == 32) return 0.0;
-  h = __funnelshift_l(m, h, c);
-  m = __funnelshift_l(l, m, c);
-  const int e = top - c + S + 1022;  // biased exponent less one: the leading bit adds it back
-  unsigned lo = __funnelshift_r(m, h, 11), hi = h >> 11;
-  const unsigned long long t = (((unsigned long long)hi << 32) | lo) + ((m >> 10) & 1u);
-  if (e < 0) return 0.0;
-  if (e >= 2046) return __hiloint2double((int)(0x7FF00000u | ((unsigned)s & 0x80000000u)), 0);
-  const unsigned long long b = t + ((unsigned long long)(unsigned)e << 52);
-  return __longlong_as_double((long long)(b | ((unsigned long long)((unsigned)s & 0x80000000u) << 32)));
-}
 
 // ------------------------------------------------------------ transforms
 template <bool INV, int R>
@@ -528,17 +401,8 @@ __device__ __forceinline__ void row_w_body(const RowArgs& a, const Pw& pw, const
 }
 
 // ------------------------------------------------------------ direct sums
-// Fixed point of 55 bits and its 28-bit limbs: v = h 2^28 + l, l in [-2^27, 2^27).
-__device__ __forceinline__ long long i64_of_f64(double x, int S) {
-  const w96 v = w_of_f64(x, S);
-  return (long long)(((unsigned long long)v.m << 32) | v.l);
-}
-__device__ __forceinline__ int2 limbs28(long long v) {
-  const int h = (int)((v + (1LL << 27)) >> 28);
-  return make_int2(h, (int)(v - ((long long)h << 28)));
-}
-constexpr int kLimbBits = 55;    // |data|, |twiddle| < 2^55: |h|, |l| <= 2^27
-constexpr int kLimbTerms = 128;  // products per 64-bit accumulator (below 2^62), then flushed
+constexpr int kDftLow = 28, kDftBits = 55;  // |data|, |twiddle| < 2^55 in limb pairs of 28 low bits
+constexpr int kDftTerms = 128;              // products per 64-bit accumulator (below 2^62), then flushed
 
 // Twiddle q (cos, -sin of 2 pi q / N) in 28-bit limbs of Q55, from the shared
 // table or (rows too long for one) from the plan's Q61 table.
@@ -546,7 +410,7 @@ template <bool GTAB>
 __device__ __forceinline__ int4 dft_twiddle(const int4* tab, const FxW* __restrict__ twfx, int q) {
   if constexpr (!GTAB) return tab[q];
   const FxW w = fx_ldw(&twfx[q]);
-  const int2 c = limbs28((((long long)w.ch << 31) + w.cl + 32) >> 6), s = limbs28((((long long)w.sh << 31) + w.sl + 32) >> 6);
+  const int2 c = limbs<kDftLow>((((long long)w.ch << 31) + w.cl + 32) >> 6), s = limbs<kDftLow>((((long long)w.sh << 31) + w.sl + 32) >> 6);
   return make_int4(c.x, c.y, s.x, s.y);
 }
 
@@ -559,11 +423,11 @@ __device__ __forceinline__ void dft_sums(const int4* __restrict__ d, int ld, int
   for (int f = 0; f < FT; ++f) C[f] = S[f] = w96{0u, 0u, 0};
   int e = 0;
 #pragma unroll 1
-  for (int j0 = 1; j0 <= J; j0 += kLimbTerms) {
+  for (int j0 = 1; j0 <= J; j0 += kDftTerms) {
     long long chh[FT], cx[FT], shh[FT], sx[FT];
 #pragma unroll
     for (int f = 0; f < FT; ++f) chh[f] = cx[f] = shh[f] = sx[f] = 0LL;
-    const int j1 = min(J + 1, j0 + kLimbTerms);
+    const int j1 = min(J + 1, j0 + kDftTerms);
 #pragma unroll 2
     for (int j = j0; j < j1; ++j) {
       e += i;
@@ -580,8 +444,8 @@ __device__ __forceinline__ void dft_sums(const int4* __restrict__ d, int ld, int
     }
 #pragma unroll
     for (int f = 0; f < FT; ++f) {
-      C[f] = w_add(C[f], w_add(w_shl64(chh[f], 28), w_shl64(cx[f], 0)));
-      S[f] = w_add(S[f], w_add(w_shl64(shh[f], 28), w_shl64(sx[f], 0)));
+      C[f] = w_add(C[f], limb_total<kDftLow>(chh[f], cx[f]));
+      S[f] = w_add(S[f], limb_total<kDftLow>(shh[f], sx[f]));
     }
   }
 }
@@ -632,7 +496,7 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
       if (mx) atomicMax(&sc.key[f], mx);
     }
     __syncthreads();
-    constexpr int fb = kLimbBits;
+    constexpr int fb = kDftBits;
     if (tid < NIN) sc.S[tid] = f64_key_exp(sc.key[tid]) - fb;
     __syncthreads();
     constexpr int FT = dft_fields<NIN>();
@@ -641,7 +505,7 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
       for (int idx = tid; idx < ng * (L + 1); idx += T) {
         const int q = idx / ng, f = idx - q * ng;
         const double2 v = load(g0 + f, q);
-        const int2 re = limbs28(i64_of_f64(v.x, sc.S[g0 + f])), im = limbs28(i64_of_f64(v.y, sc.S[g0 + f]));
+        const int2 re = limbs<kDftLow>(i64_of_f64(v.x, sc.S[g0 + f])), im = limbs<kDftLow>(i64_of_f64(v.y, sc.S[g0 + f]));
         data[f * ld + q] = make_int4(re.x, re.y, im.x, im.y);
       }
       __syncthreads();
@@ -653,10 +517,10 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
         dft_sums<FT, GTAB>(d, ld, L, k, N, tab, twfx, C, S);
 #pragma unroll
         for (int u = 0; u < FT; ++u) {
-          const int f = g0 + s * FT + u, e = sc.S[f] - 27;
+          const int f = g0 + s * FT + u, e = sc.S[f] - (kDftBits - kDftLow);
           const bool bad = sc.key[f] >= kNonFinite;
           const int4 v0 = d[u * ld];
-          const w96 V0 = w_shl64(((long long)v0.x << 28) + v0.y, 27);
+          const w96 V0 = w_shl64(((long long)v0.x << kDftLow) + v0.y, kDftBits - kDftLow);
           const w96 p = w_add(C[u], S[u]), r = w_sub(C[u], S[u]);
           grid[f * N + k] = bad ? nan : f64_of_w(w_add(V0, w_add(p, p)), e);
           if (k > 0 && N - k > k) grid[f * N + N - k] = bad ? nan : f64_of_w(w_add(V0, w_add(r, r)), e);
@@ -689,7 +553,7 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
 
   if constexpr (OUT_MODE == kOutG) {
     constexpr int FT = dft_fields<NOUT>();
-    constexpr int fb = kLimbBits - 1;  // pairs x_j +- x_{N-j} take one bit more
+    constexpr int fb = kDftBits - 1;  // pairs x_j +- x_{N-j} take one bit more
     for (int f = tid >> 5; f < NOUT; f += T >> 5) {
       unsigned mx = 0u;
       for (int k = tid & 31; k < N; k += 32) mx = max(mx, f64_key(grid[f * N + k]));
@@ -711,11 +575,11 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
         int2 p, r;
         if (i > 0) {
           const long long Y = i64_of_f64(x[N - i], S);
-          p = limbs28(X + Y);
-          r = limbs28(X - Y);
+          p = limbs<kDftLow>(X + Y);
+          r = limbs<kDftLow>(X - Y);
         } else {  // x_0 and, for an even row, the point opposite
-          p = limbs28(X);
-          r = limbs28(N % 2 == 0 ? i64_of_f64(x[half], S) : 0LL);
+          p = limbs<kDftLow>(X);
+          r = limbs<kDftLow>(N % 2 == 0 ? i64_of_f64(x[half], S) : 0LL);
         }
         data[f * ld + i] = make_int4(p.x, p.y, r.x, r.y);
       }
@@ -727,10 +591,10 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
         dft_sums<FT, GTAB>(d, ld, J, q % N, N, tab, twfx, C, S);
 #pragma unroll
         for (int u = 0; u < FT; ++u) {
-          const int f = g0 + s * FT + u, e = sc.S[f] - 27;
+          const int f = g0 + s * FT + u, e = sc.S[f] - (kDftBits - kDftLow);
           const int4 v0 = d[u * ld];
-          const long long x0 = ((long long)v0.x << 28) + v0.y, xh = ((long long)v0.z << 28) + v0.w;
-          const w96 re = w_add(C[u], w_shl64(x0 + (q & 1 ? -xh : xh), 27));
+          const long long x0 = ((long long)v0.x << kDftLow) + v0.y, xh = ((long long)v0.z << kDftLow) + v0.w;
+          const w96 re = w_add(C[u], w_shl64(x0 + (q & 1 ? -xh : xh), kDftBits - kDftLow));
           const bool bad = sc.key[f] >= kNonFinite;
           block[(long)q * sq + f] =
               bad ? make_double2(nan, nan) : make_double2(wj * f64_of_w(re, e), wj * f64_of_w(S[u], e));
