@@ -179,26 +179,38 @@ struct Rk4 {
   double2* ystage;  // stage input for the next stage
   double2* acc;     // k1 + 2 k2 + 2 k3
   double2* tend;    // mode 0 output
-  __device__ void apply(long i, double2 k) const {
+  struct In {
+    double2 y, a;  // y0 and acc at a slot
+  };
+  // An epilogue of several fields reads all of them before its first store
+  // (which the compiler cannot move a later load across).
+  __device__ In ld(long i) const {
+    In r{};
+    if (mode > 0) r.y = y0[i];
+    if (mode > 1) r.a = acc[i];
+    return r;
+  }
+  __device__ void apply(long i, double2 k) const { apply(i, k, ld(i)); }
+  __device__ void apply(long i, double2 k, const In& in) const {
     if (mode == 0) {
       tend[i] = k;
     } else if (mode == 1) {
       acc[i] = k;
-      ystage[i] = cadd(y0[i], cscale(0.5 * dt, k));
+      ystage[i] = cadd(in.y, cscale(0.5 * dt, k));
     } else if (mode == 2) {
-      acc[i] = cadd(acc[i], cscale(2.0, k));
-      ystage[i] = cadd(y0[i], cscale(0.5 * dt, k));
+      acc[i] = cadd(in.a, cscale(2.0, k));
+      ystage[i] = cadd(in.y, cscale(0.5 * dt, k));
     } else if (mode == 3) {
-      acc[i] = cadd(acc[i], cscale(2.0, k));
-      ystage[i] = cadd(y0[i], cscale(dt, k));
+      acc[i] = cadd(in.a, cscale(2.0, k));
+      ystage[i] = cadd(in.y, cscale(dt, k));
     } else {
-      y0[i] = cadd(y0[i], cscale(dt / 6.0, cadd(acc[i], k)));
+      y0[i] = cadd(in.y, cscale(dt / 6.0, cadd(in.a, k)));
     }
   }
   __device__ void zero(long i) const {
     const double2 z = make_double2(0.0, 0.0);
     if (mode == 0) tend[i] = z;
-    else if (mode < 4) { acc[i] = z; ystage[i] = z; }
+    else if (mode < 4) ystage[i] = z;  // acc is read at l >= m only
     else y0[i] = z;
   }
 };
@@ -553,6 +565,7 @@ struct SweEpi {
     }
     const double2 a0 = tr ? z0 : an[0], a1 = tr ? z0 : an[1], a2 = tr ? z0 : an[2], a3 = tr ? z0 : an[3];
     const double2 zs = state[base], ds = state[base + n2], ps = state[base + 2 * n2];
+    const Rk4::In i0 = rk.ld(base), i1 = rk.ld(base + n2), i2 = rk.ld(base + 2 * n2);
     const double lap = s.lap(l);
     double2 k0 = a0;
     double2 k1 = csub(a1, cscale(lap, cadd(a2, ps)));
@@ -570,9 +583,9 @@ struct SweEpi {
     }
     if (forcing) k2 = cadd(k2, forcing[2 * n2 + fo]);  // after it, as -nu4 lap^2 phi_s
     if (l == 0) k0 = k1 = k2 = z0;
-    rk.apply(base, k0);
-    rk.apply(base + n2, k1);
-    rk.apply(base + 2 * n2, k2);
+    rk.apply(base, k0, i0);
+    rk.apply(base + n2, k1, i1);
+    rk.apply(base + 2 * n2, k2, i2);
   }
   __device__ void zero(int b, int l, int m) const {
     const long n2 = (long)(s.L + 1) * (s.L + 1);
