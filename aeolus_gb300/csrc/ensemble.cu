@@ -163,8 +163,7 @@ __global__ void __launch_bounds__(256) g_slice_synth(Grouped<SliceSynthArg<Deriv
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
   const SliceSynthArg<Derive>& a = g.arg[k];
-  split_synth_slice_body<Derive>(a.dm, a.kcum, a.batch, a.mb, a.d, a.digits, a.ecol, loc % g.gx[k], loc / g.gx[k],
-                                 g.gy[k]);
+  split_synth_slice_body<Derive>(a.dm, a.kcum, a.batch, a.mb, a.d, a.digits, a.ecol, loc % g.gx[k], loc / g.gx[k]);
 }
 
 template <int NF>
@@ -173,8 +172,7 @@ __global__ void __launch_bounds__(256) g_slice_anal(Grouped<SliceAnalArg> g) {
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
   const SliceAnalArg& a = g.arg[k];
-  split_anal_slice_body<NF>(a.dm, a.batch, a.mb, a.nblk, a.FG, a.digits, a.ecol, loc % g.gx[k], loc / g.gx[k],
-                            g.gy[k]);
+  split_anal_slice_body<NF>(a.dm, a.batch, a.mb, a.nblk, a.FG, a.digits, a.ecol, loc % g.gx[k], loc / g.gx[k]);
 }
 
 // Persistent tensor-core tiles of all groups in one list.

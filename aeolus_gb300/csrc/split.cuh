@@ -268,12 +268,15 @@ __device__ inline void store_digits8(__nv_bfloat16* tile, int r, int k0, const l
 }
 
 // ------------------------------------------------- synthesis data slicing
-// grid (m, member chunk of `mb` members); columns (b, f, re/im).
+// grid (m, member chunk of `mb` members); columns (b, f, re/im).  The columns
+// that pad the last tile are not written: a column's accumulators depend on
+// that column alone, and no epilogue writes those of a column past the last
+// (zeroing them took a third of the slicing time of one member).
 template <class Derive>
 __device__ __forceinline__ void split_synth_slice_body(const SplitDims& dm, const long long* __restrict__ kcum,
                                                        int batch, int mb, const Derive& der,
                                                        __nv_bfloat16* __restrict__ dsyn, int* __restrict__ ecol,
-                                                       int bx, int by, int gy) {
+                                                       int bx, int by) {
   constexpr int NF = Derive::NF;
   extern __shared__ double s_val[];  // [mb*NF*2][ks]
   __shared__ int s_exp[256];
@@ -345,16 +348,6 @@ __device__ __forceinline__ void split_synth_slice_body(const SplitDims& dm, cons
     }
     store_digits8(dsyn + dsyn_tile(kcum, dm, m, n / kNT), n % kNT, t0, X);
   }
-  if (by == gy - 1) {  // zero the columns that pad the last tile
-    const int n0 = batch * NF * 2, n1 = dm.ntiles * kNT;
-    for (int idx = threadIdx.x; idx < (n1 - n0) * Kp; idx += blockDim.x) {
-      const int n = n0 + idx / Kp, t = idx % Kp;
-      __nv_bfloat16* tile = dsyn + dsyn_tile(kcum, dm, m, n / kNT);
-#pragma unroll
-      for (int s = 0; s < kSlices; ++s) tile[tile_elem(kNT, s, n % kNT, t)] = __float2bfloat16(0.0f);
-      if (t == 0) ecol[(long long)m * dm.ntiles * kNT + n] = 0;
-    }
-  }
 }
 
 // Four CTAs per SM (64 registers) for the FP64 derives; three (85) for the
@@ -365,7 +358,7 @@ __global__ void __launch_bounds__(256, DeriveHasDf<Derive>::value ? 3 : 4) split
                                                                __nv_bfloat16* __restrict__ dsyn,
                                                                int* __restrict__ ecol) {
   pdl_wait();
-  split_synth_slice_body<Derive>(dm, kcum, batch, mb, der, dsyn, ecol, blockIdx.x, blockIdx.y, gridDim.y);
+  split_synth_slice_body<Derive>(dm, kcum, batch, mb, der, dsyn, ecol, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------- analysis data slicing
@@ -377,7 +370,7 @@ __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
 template <int NF>
 __device__ __forceinline__ void split_anal_slice_body(const SplitDims& dm, int batch, int mb, int nblk,
                                                       const long long* __restrict__ FG, __nv_bfloat16* __restrict__ dana,
-                                                      int* __restrict__ ecol, int bx, int by, int gy) {
+                                                      int* __restrict__ ecol, int bx, int by) {
   extern __shared__ long long s_wval[];  // [mb*NF*2][ns]
   __shared__ int s_exp[256];
   const int m = bx, L = dm.L, nlat = dm.nlat, NK = dm.NK;
@@ -419,16 +412,6 @@ __device__ __forceinline__ void split_anal_slice_body(const SplitDims& dm, int b
     for (int u = 0; u < 8; ++u) X[u] = j0 + u < nlat ? pk_align(s_wval[c * ns + j0 + u], S) : 0LL;
     store_digits8(dana + dana_tile(dm, m, n / kNT), n % kNT, j0, X);
   }
-  if (by == gy - 1) {
-    const int n0 = batch * NF * 2, n1 = dm.ntiles * kNT;
-    for (int idx = threadIdx.x; idx < (n1 - n0) * NK; idx += blockDim.x) {
-      const int n = n0 + idx / NK, j = idx % NK;
-      __nv_bfloat16* tile = dana + dana_tile(dm, m, n / kNT);
-#pragma unroll
-      for (int s = 0; s < kSlices; ++s) tile[tile_elem(kNT, s, n % kNT, j)] = __float2bfloat16(0.0f);
-      if (j == 0) ecol[(long long)m * dm.ntiles * kNT + n] = 0;
-    }
-  }
 }
 
 constexpr int kAnalSliceThreads = 128;  // 8 CTAs per SM: more G loads in flight per SM
@@ -438,7 +421,7 @@ __global__ void __launch_bounds__(kAnalSliceThreads, 8) split_anal_slice_kernel(
                                                               __nv_bfloat16* __restrict__ dana,
                                                               int* __restrict__ ecol) {
   pdl_wait();
-  split_anal_slice_body<NF>(dm, batch, mb, nblk, FG, dana, ecol, blockIdx.x, blockIdx.y, gridDim.y);
+  split_anal_slice_body<NF>(dm, batch, mb, nblk, FG, dana, ecol, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------- tensor-core kernels
@@ -994,6 +977,11 @@ SplitParts split_synth_parts(const aeolus_plan_impl* p, int batch, void* scratch
   r.ecol = reinterpret_cast<int*>(w);
   // 32 KB of staged values: four 256-thread CTAs per SM (64 registers each)
   r.mb = slice_members(NF, r.dm.L + 2, p->tune_slice_mb, 32 * 1024);
+  // fewer members per CTA while that leaves at most one wave (12.3 -> 8.4 us
+  // for 4 members at l_max 85, 12.9 -> 8.2 for 16 at 42; past one wave it costs:
+  // 19 -> 23 us for 8 at 127)
+  if (p->tune_slice_mb <= 0)
+    while (r.mb > 1 && (long)(r.dm.L + 1) * ((batch + r.mb - 2) / (r.mb - 1)) <= 4L * p->sm_count) --r.mb;
   r.smem = (size_t)r.mb * NF * 2 * ((r.dm.L + 1) | 1) * 8;
   r.grid = dim3(r.dm.L + 1, (batch + r.mb - 1) / r.mb);
   return r;
@@ -1007,7 +995,12 @@ SplitParts split_anal_parts(const aeolus_plan_impl* p, int batch, void* scratch,
   r.digits = reinterpret_cast<__nv_bfloat16*>(w);
   w += align256((size_t)(r.dm.L + 1) * r.dm.ntiles * kSlices * kNT * r.dm.NK * 2);
   r.ecol = reinterpret_cast<int*>(w);
-  r.mb = slice_members(NF, r.dm.nlat + 1, p->tune_slice_mb_anal);
+  // eight columns per CTA (the digits of eight neighbouring columns fill whole
+  // 128-byte lines), so that eight CTAs of staged loads share an SM: 14.6 -> 7.8
+  // us for 8 members and 50.9 -> 38.8 us for 64 (l_max 127, 4 fields, against 64 KB
+  // of staged words per CTA), 25.5 -> 22.5 us with 9 fields
+  r.mb = p->tune_slice_mb_anal > 0 ? slice_members(NF, r.dm.nlat + 1, p->tune_slice_mb_anal)
+                                   : std::min(slice_members(NF, r.dm.nlat + 1, 0), std::max(1, 4 / NF));
   r.smem = (size_t)r.mb * NF * 2 * (r.dm.nlat | 1) * 8;
   r.grid = dim3(top + 1, (batch + r.mb - 1) / r.mb);
   return r;
