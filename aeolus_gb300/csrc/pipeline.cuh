@@ -159,17 +159,31 @@ int launch_rows_fx(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, cu
   return AEOLUS_OK;
 }
 
+// At most two row CTAs per SM: 320 threads instead of 128 shorten every phase
+// of a row (each pass of 9 fields then takes one or two rounds).  Tendency
+// chains only, whose rows have the most phases.  SWE RK4 per stage: 47.2 ->
+// 43.9 us at one CTA per SM (l_max 85, one member), 56.8 -> 54.4 at two; from
+// three on it costs (86.6 -> 90.8 us at 3.8 per SM).
+template <int IN_MODE, int OUT_MODE>
+inline bool split_few_rows(const aeolus_plan_impl* p, dim3 grid) {
+  return IN_MODE == kInF && OUT_MODE == kOutG && (long)grid.x * grid.y <= 2L * p->sm_count;
+}
+template <int IN_MODE, int OUT_MODE>
+constexpr int few_row_threads() { return IN_MODE == kInF && OUT_MODE == kOutG ? kFewRowThreads : kFx8Threads; }
+
 // Fixed radix sequence (R0, 8, 8): compile-time lengths, kFx8Threads threads
 // (the plan's row-thread knob does not apply).
 template <class Pw, int IN_MODE, int OUT_MODE, int R0>
 int launch_rows_fx8(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, cudaStream_t st) {
   const size_t sm = row_fx8_smem_bytes<Pw>(R0);
-  auto kern = row_kernel_fx8<Pw, IN_MODE, OUT_MODE, R0>;
+  const dim3 grid(p->nlat, a.batch);
+  const bool few = split_few_rows<IN_MODE, OUT_MODE>(p, grid);
+  auto kern = few ? row_kernel_fx8<Pw, IN_MODE, OUT_MODE, R0, few_row_threads<IN_MODE, OUT_MODE>()> : row_kernel_fx8<Pw, IN_MODE, OUT_MODE, R0, kFx8Threads>;
   int s = allow_smem(kern, sm);
   if (s) return s;
   ProfScope prof(IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_fx_c2r_products_r2c" : "rows_fx_c2r") : "rows_fx_r2c",
                  st);
-  launch_pdl(kern, dim3(p->nlat, a.batch), dim3(kFx8Threads), sm, st, a, pw, static_cast<const FxW*>(p->twfx),
+  launch_pdl(kern, grid, dim3(few ? kFewRowThreads : kFx8Threads), sm, st, a, pw, static_cast<const FxW*>(p->twfx),
              fx_consts());
   AE_LAUNCH("row_kernel_fx8");
   return AEOLUS_OK;
@@ -180,12 +194,14 @@ int launch_rows_fx8(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, c
 template <class Pw, int IN_MODE, int OUT_MODE, class S>
 int launch_rows_pfa(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, cudaStream_t st) {
   const size_t sm = row_pfa_smem_bytes<Pw, S>();
-  auto kern = row_kernel_pfa<Pw, IN_MODE, OUT_MODE, S>;
+  const dim3 grid = row_pfa_grid<Pw>(p->nlat, a.batch);
+  const bool few = split_few_rows<IN_MODE, OUT_MODE>(p, grid);
+  auto kern = few ? row_kernel_pfa<Pw, IN_MODE, OUT_MODE, S, few_row_threads<IN_MODE, OUT_MODE>()> : row_kernel_pfa<Pw, IN_MODE, OUT_MODE, S, kPfaThreads>;
   int s = allow_smem(kern, sm);
   if (s) return s;
   ProfScope prof(IN_MODE == kInF ? (OUT_MODE == kOutG ? "rows_fx_c2r_products_r2c" : "rows_fx_c2r") : "rows_fx_r2c",
                  st);
-  launch_pdl(kern, row_pfa_grid<Pw>(p->nlat, a.batch), dim3(kPfaThreads), sm, st, a, pw,
+  launch_pdl(kern, grid, dim3(few ? kFewRowThreads : kPfaThreads), sm, st, a, pw,
              static_cast<const FxW*>(p->twfx), fx_consts());
   AE_LAUNCH("row_kernel_pfa");
   return AEOLUS_OK;
@@ -248,7 +264,8 @@ WideRowCfg wide_row_cfg(const aeolus_plan_impl* p, int batch) {
     }
     c.smem = row_w_smem_bytes<Pw>(f, c.nr);
     // few rows: twice the threads shorten each row; otherwise more CTAs per SM
-    if ((long)c.grid.x * c.grid.y <= 2L * p->sm_count) c.threads = 256;
+    if ((long)c.grid.x * c.grid.y <= 1L * p->sm_count) c.threads = 512;
+    else if ((long)c.grid.x * c.grid.y <= 2L * p->sm_count) c.threads = 256;
   } else {
     c.gf = row_w_dft_group<Pw>(f, p->lmax);
     c.gtab = row_w_dft_smem<Pw>(f, p->lmax, c.gf, false) > 220 * 1024;
@@ -256,7 +273,7 @@ WideRowCfg wide_row_cfg(const aeolus_plan_impl* p, int batch) {
     const int items = (std::min(c.gf, Pw::NIN) + dft_fields<Pw::NIN>() - 1) / dft_fields<Pw::NIN>() * (f.N / 2 + 1);
     c.threads = 32 * leg_warps((items + 31) / 32);
   }
-  if (p->tune_row_threads > 0) c.threads = std::min(p->tune_row_threads, kWideMaxThreads);
+  if (p->tune_row_threads > 0) c.threads = std::min(p->tune_row_threads, 256);
   return c;
 }
 

@@ -530,6 +530,8 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
 //  * the digit reversal of the in-place DIT input is arithmetic:
 //    natural index q = 64 t0 + 8 t1 + t2 sits at t0 + R0 (t1 + 8 t2).
 constexpr int kFx8Threads = 128;
+// Threads of a row CTA where the rows are too few to fill the SMs (row_threads_split).
+constexpr int kFewRowThreads = 320;
 
 template <int R0>
 struct Fx8 {
@@ -541,14 +543,14 @@ struct Fx8 {
   static __device__ __forceinline__ int rev(int q) { return (q >> 6) + R0 * (((q >> 3) & 7) + 8 * (q & 7)); }
 };
 
-template <int R0, bool INV, int R, int LS, bool DIT, bool TW, bool CONV, int NFLD>
+template <int T, int R0, bool INV, int R, int LS, bool DIT, bool TW, bool CONV, int NFLD>
 __device__ __forceinline__ void fx8_stage(cfx* __restrict__ x, const FxW* __restrict__ tw, const FxConst& kc,
                                           const float* sqa, const float* sqb) {
   using Row = Fx8<R0>;
   constexpr int n = Row::n, nb = n / R, NS = LS * R, stride = n / NS, G = nb / LS;
   constexpr bool kmajor = R0 == 3 && LS == R0;
 #pragma unroll 1
-  for (int idx = threadIdx.x; idx < NFLD * nb; idx += kFx8Threads) {
+  for (int idx = threadIdx.x; idx < NFLD * nb; idx += T) {
     int f, g, k;
     if constexpr (kmajor) {
       g = idx % G;
@@ -592,33 +594,33 @@ __device__ __forceinline__ void fx8_stage(cfx* __restrict__ x, const FxW* __rest
 
 // In-place inverse (DIT, digit-reversed input) or forward (DIF, with the
 // double-float rows rounded to fixed point by its first stage) transforms.
-template <int R0, bool INV, int NFLD>
+template <int T, int R0, bool INV, int NFLD>
 __device__ __forceinline__ void fx8_fft(cfx* x, const FxW* __restrict__ tw, const FxConst& kc, const float* sqa,
                                         const float* sqb) {
   if constexpr (INV) {
-    fx8_stage<R0, true, R0, 1, true, false, false, NFLD>(x, tw, kc, nullptr, nullptr);
+    fx8_stage<T, R0, true, R0, 1, true, false, false, NFLD>(x, tw, kc, nullptr, nullptr);
     __syncthreads();
-    fx8_stage<R0, true, 8, R0, true, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
+    fx8_stage<T, R0, true, 8, R0, true, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
     __syncthreads();
-    fx8_stage<R0, true, 8, 8 * R0, true, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
+    fx8_stage<T, R0, true, 8, 8 * R0, true, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
     __syncthreads();
   } else {
-    fx8_stage<R0, false, 8, 8 * R0, false, true, true, NFLD>(x, tw, kc, sqa, sqb);
+    fx8_stage<T, R0, false, 8, 8 * R0, false, true, true, NFLD>(x, tw, kc, sqa, sqb);
     __syncthreads();
-    fx8_stage<R0, false, 8, R0, false, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
+    fx8_stage<T, R0, false, 8, R0, false, true, false, NFLD>(x, tw, kc, nullptr, nullptr);
     __syncthreads();
-    fx8_stage<R0, false, R0, 1, false, false, false, NFLD>(x, tw, kc, nullptr, nullptr);
+    fx8_stage<T, R0, false, R0, 1, false, false, false, NFLD>(x, tw, kc, nullptr, nullptr);
     __syncthreads();
   }
 }
 
-template <class Pw, int IN_MODE, int OUT_MODE, int R0>
+template <class Pw, int IN_MODE, int OUT_MODE, int R0, int T = kFx8Threads>
 __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, const FxW* __restrict__ twfx,
                                              const FxConst& kc, int bx, int by) {
   using Row = Fx8<R0>;
   constexpr int NIN = Pw::NIN, NOUT = Pw::NOUT;
   constexpr int NF = NIN > NOUT ? NIN : NOUT;
-  constexpr int n = Row::n, N = Row::N, fs = Row::fs, hb = Row::hb, T = kFx8Threads;
+  constexpr int n = Row::n, N = Row::N, fs = Row::fs, hb = Row::hb;
   // (order, field) passes: stride PS, a multiple of the field count
   constexpr int PSI = (T / NIN) * NIN, QSI = T / NIN;
   constexpr int PSO = (T / NOUT) * NOUT, QSO = T / NOUT;
@@ -697,7 +699,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
       }
     }
     __syncthreads();
-    fx8_fft<R0, true, NIN>(buf0, twfx, kc, nullptr, nullptr);
+    fx8_fft<T, R0, true, NIN>(buf0, twfx, kc, nullptr, nullptr);
   } else {
     df* x0 = reinterpret_cast<df*>(buf0);
     for (int idx = tid; idx < NIN * N; idx += T) {
@@ -729,8 +731,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
       }
     }
 #pragma unroll 1
-    for (int it = 0; it < N / T; ++it) {
-      const int k = tid + it * T;
+    for (int k = tid; k < N; k += T) {
       const int slot = 2 * Row::swz(k >> 1) + (k & 1);
       df in[NIN], out[NOUT];
 #pragma unroll
@@ -772,7 +773,7 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
       fx_pow2_split(-S, s_pa[tid], s_pb[tid]);
     }
     __syncthreads();
-    fx8_fft<R0, false, NOUT>(buf0, twfx, kc, s_pa, s_pb);
+    fx8_fft<T, R0, false, NOUT>(buf0, twfx, kc, s_pa, s_pb);
     if (tid < PSO) {
       const int f = tid % NOUT;
       const int e = s_in[f] - 1;  // R2 / 2 in units of 2^S
@@ -790,11 +791,11 @@ __device__ __forceinline__ void row_fx8_body(const RowArgs& a, const Pw& pw, con
   }
 }
 
-template <class Pw, int IN_MODE, int OUT_MODE, int R0>
-__global__ void __launch_bounds__(kFx8Threads, 6) row_kernel_fx8(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
-                                                                 FxConst kc) {
+template <class Pw, int IN_MODE, int OUT_MODE, int R0, int T>
+__global__ void __launch_bounds__(T, T == kFx8Threads ? 6 : 2) row_kernel_fx8(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
+                                                                              FxConst kc) {
   pdl_wait();
-  row_fx8_body<Pw, IN_MODE, OUT_MODE, R0>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
+  row_fx8_body<Pw, IN_MODE, OUT_MODE, R0, T>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
 }
 
 template <class Pw>

@@ -130,14 +130,14 @@ struct PwHasPairs<Pw, std::void_t<decltype(&Pw::df_op2)>> : std::true_type {};
 // PASS1 then the strided pass, the forward the strided pass then PASS1.
 // CONV: the rows still hold double-floats, rounded to the field's fixed-
 // point scale (pa pb = 2^-S) as they are loaded.
-template <class S, bool INV, bool PASS1, bool CONV, int NFLD, int NPER, int RS>
+template <int T, class S, bool INV, bool PASS1, bool CONV, int NFLD, int NPER, int RS>
 __device__ __forceinline__ void pfa_pass(cfx* __restrict__ x, const FxW* __restrict__ tw, const FxConst& kc,
                                          const float* sqa, const float* sqb) {
   constexpr int R = PASS1 ? S::R2 : S::R1;        // butterfly radix
   constexpr int NB = PASS1 ? S::R1 : S::R2;       // butterflies per block
   constexpr int TWS = 2 * S::R0;                  // w_P = w_N^(N / P)
 #pragma unroll 1
-  for (int idx = threadIdx.x; idx < NFLD * S::R0 * NB; idx += kPfaThreads) {
+  for (int idx = threadIdx.x; idx < NFLD * S::R0 * NB; idx += T) {
     // f: (member row, field) pair, NPER fields of each row's RS slots
     const int f = idx / (S::R0 * NB), rem = idx - f * (S::R0 * NB), r = rem / NB, k = rem - r * NB;
     cfx* y = x + (NFLD == NPER ? f * S::fs : (f / NPER) * RS + (f % NPER) * S::fs) + r * S::P;
@@ -222,14 +222,14 @@ struct alignas(16) PfaCtaScratch {
   df wj;
 };
 
-template <class Pw, int IN_MODE, int OUT_MODE, class S>
+template <class Pw, int IN_MODE, int OUT_MODE, class S, int T = kPfaThreads>
 __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, const FxW* __restrict__ twfx,
                                              const FxConst& kc, int bx, int by) {
   constexpr int NIN = Pw::NIN, NOUT = Pw::NOUT;
   constexpr int NF = NIN > NOUT ? NIN : NOUT;
   constexpr int NR = pfa_rows_per_cta<Pw>();
   constexpr int NRI = NR * NIN, NRO = NR * NOUT;  // (member row, field) pairs in and out
-  constexpr int n = S::n, N = S::N, fs = S::fs, hb = S::hb, P = S::P, R0 = S::R0, T = kPfaThreads;
+  constexpr int n = S::n, N = S::N, fs = S::fs, hb = S::hb, P = S::P, R0 = S::R0;
   constexpr int RS = NF * fs;  // slots of one member row
   constexpr int PSI = (T / NRI) * NRI, QSI = T / NRI;
   static_assert(NRI <= T && NRO <= T, "one thread per (row, field) for the block exponents");
@@ -347,9 +347,9 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
       }
       __syncthreads();
     }
-    pfa_pass<S, true, true, false, NRI, NIN, RS>(buf0, twfx, kc, nullptr, nullptr);
+    pfa_pass<T, S, true, true, false, NRI, NIN, RS>(buf0, twfx, kc, nullptr, nullptr);
     __syncthreads();
-    pfa_pass<S, true, false, false, NRI, NIN, RS>(buf0, twfx, kc, nullptr, nullptr);
+    pfa_pass<T, S, true, false, false, NRI, NIN, RS>(buf0, twfx, kc, nullptr, nullptr);
     __syncthreads();
   }
 
@@ -482,9 +482,9 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
       fx_pow2_split(-S0, s_pa[tid], s_pb[tid]);  // indexed by (row, output field) for the passes
     }
     __syncthreads();
-    pfa_pass<S, false, false, true, NRO, NOUT, RS>(buf0, twfx, kc, s_pa, s_pb);
+    pfa_pass<T, S, false, false, true, NRO, NOUT, RS>(buf0, twfx, kc, s_pa, s_pb);
     __syncthreads();
-    pfa_pass<S, false, true, false, NRO, NOUT, RS>(buf0, twfx, kc, nullptr, nullptr);
+    pfa_pass<T, S, false, true, false, NRO, NOUT, RS>(buf0, twfx, kc, nullptr, nullptr);
     __syncthreads();
     // radix-R0 across the blocks for the order groups c + jP and P - c + jP
     // (item 0: the self-paired groups 0 and P/2), then the real-FFT
@@ -519,11 +519,11 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
   }
 }
 
-template <class Pw, int IN_MODE, int OUT_MODE, class S>
-__global__ void __launch_bounds__(kPfaThreads, 6) row_kernel_pfa(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
-                                                                 FxConst kc) {
+template <class Pw, int IN_MODE, int OUT_MODE, class S, int T>
+__global__ void __launch_bounds__(T, T == kPfaThreads ? 6 : 2) row_kernel_pfa(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
+                                                                              FxConst kc) {
   pdl_wait();
-  row_pfa_body<Pw, IN_MODE, OUT_MODE, S>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
+  row_pfa_body<Pw, IN_MODE, OUT_MODE, S, T>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
 }
 
 template <class Pw, class S>
