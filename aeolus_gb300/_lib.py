@@ -107,6 +107,10 @@ SIGNATURES = {
                                        c_size_t, c_void_p]),
     "aeolus_swe_rk4_adjoint": (c_int, [c_void_p, POINTER(SweParams), c_void_p, c_void_p, c_int, c_double, c_void_p,
                                        c_size_t, c_void_p]),
+    "aeolus_swe_rk4_stages": (c_int, [c_void_p, POINTER(SweParams), c_void_p, c_void_p, c_void_p, c_int, c_double,
+                                      c_void_p, c_size_t, c_void_p]),
+    "aeolus_swe_rk4_adjoint_stages": (c_int, [c_void_p, POINTER(SweParams), c_void_p, c_void_p, c_void_p, c_int,
+                                              c_double, c_void_p, c_size_t, c_void_p]),
     "aeolus_ensemble_create": (c_int, [c_int, POINTER(c_void_p), POINTER(c_int), POINTER(BveParams),
                                        POINTER(c_void_p)]),
     "aeolus_ensemble_create_swe": (c_int, [c_int, POINTER(c_void_p), POINTER(c_int), POINTER(SweParams),

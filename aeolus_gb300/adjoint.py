@@ -12,31 +12,74 @@ kernels.  Every backward is a call into ``libaeolus_gb300.so``:
 * :func:`swe_rk4_checkpointed` / :func:`bve_rk4_checkpointed` advance
   ``nsteps`` RK4 steps and keep the step input every ``every`` steps; their
   backward re-runs each segment forward from its checkpoint (holding the
-  ``every`` step inputs of one segment) and applies the per-step adjoint
-  (``aeolus_swe_rk4_adjoint``), which recomputes the stage inputs and runs
-  the four tendency VJPs on the device.
+  ``every`` step inputs of one segment) and applies the per-step adjoint,
+  which runs the four tendency VJPs on the device.  The shallow-water path
+  keeps the stage inputs of a segment too, as long as they fit into the size
+  of one step adjoint's workspace (``aeolus_swe_rk4_adjoint_stages``; beyond
+  that the step adjoint recomputes them), and the last segment, with which the
+  backward starts, from the forward pass.
 
-Peak device memory is therefore (checkpoints + one segment) states plus one
-RK4-adjoint workspace, independent of ``nsteps``.
+Peak device memory is therefore (checkpoints + two segments) states plus
+three RK4-adjoint workspaces at most, independent of ``nsteps``.
 """
 from __future__ import annotations
 
 import torch
 
-from .ops import bve_rk4_adjoint, swe_rk4_adjoint
+from . import _lib
+from .ops import bve_rk4_adjoint, swe_rk4_adjoint, swe_rk4_adjoint_stages, swe_rk4_stages
+
+
+def _swe_args(m):
+    return m._plan.id, m.R, m.Omega, m.gravity, m.mean_depth, m.nu4
+
+
+def _stage_steps(m, y, every):
+    """Steps of a segment whose stage inputs (three states each) are kept: as
+    many as fit into the size of one step adjoint's workspace."""
+    L = m._plan.lmax
+    members = y.numel() // (3 * (L + 1) * (L + 1))
+    if members == 0:
+        return 0
+    return min(every, m._plan.workspace_bytes(_lib.OP_SWE_RK4_ADJOINT, members) // (3 * 16 * y.numel()))
+
+
+def _swe_segment(m, y, dt, n, keep, last):
+    """[(input, stage inputs or None)] of n steps from y, and with `last` the
+    state after them."""
+    steps = []
+    for i in range(n):
+        step = last or i < n - 1
+        nxt, stages = None, None
+        if i < keep:
+            nxt, stages = swe_rk4_stages(*_swe_args(m), y, dt, m.forcing, step)
+        elif step:
+            nxt = m.rk4(y, dt, 1, check=False)
+        steps.append((y, stages))
+        y = nxt
+    return steps, y
 
 
 class _SweRk4Checkpointed(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y0, model, dt, nsteps, every):
         every = max(1, int(every))
+        nsteps = int(nsteps)
         ckpts = []
         y = y0.detach()
-        for i in range(nsteps):
+        # the backward starts with the last segment: its steps keep their
+        # inputs from here on instead of being run again
+        head = (nsteps - 1) // every * every if ctx.needs_input_grad[0] and nsteps > 0 else nsteps
+        for i in range(head):
             if i % every == 0:
                 ckpts.append(y.clone())
             y = model.rk4(y, dt, 1, check=False)
-        ctx.model, ctx.dt, ctx.nsteps, ctx.every, ctx.ckpts = model, float(dt), int(nsteps), every, ckpts
+        ctx.keep, ctx.tail = 0, []
+        if head < nsteps:
+            ckpts.append(y.clone())
+            ctx.keep = _stage_steps(model, y, every)
+            ctx.tail, y = _swe_segment(model, ckpts[-1], float(dt), nsteps - head, ctx.keep, True)
+        ctx.model, ctx.dt, ctx.nsteps, ctx.every, ctx.ckpts = model, float(dt), nsteps, every, ckpts
         return y
 
     @staticmethod
@@ -44,14 +87,16 @@ class _SweRk4Checkpointed(torch.autograd.Function):
         m = ctx.model
         yb = ybar.contiguous()
         for seg in range(len(ctx.ckpts) - 1, -1, -1):
-            start = seg * ctx.every
-            n = min(ctx.every, ctx.nsteps - start)
-            states = [ctx.ckpts[seg]]
-            for _ in range(n - 1):
-                states.append(m.rk4(states[-1], ctx.dt, 1, check=False))
-            for i in range(n - 1, -1, -1):
-                yb = swe_rk4_adjoint(m._plan.id, m.R, m.Omega, m.gravity, m.mean_depth, m.nu4, states[i], yb, ctx.dt,
-                                     m.forcing)
+            if seg == len(ctx.ckpts) - 1:
+                steps = list(ctx.tail)
+            else:
+                steps, _ = _swe_segment(m, ctx.ckpts[seg], ctx.dt, ctx.every, ctx.keep, False)
+            while steps:
+                y, stages = steps.pop()
+                if stages is None:
+                    yb = swe_rk4_adjoint(*_swe_args(m), y, yb, ctx.dt, m.forcing)
+                else:
+                    yb = swe_rk4_adjoint_stages(*_swe_args(m), y, stages, yb, ctx.dt, m.forcing)
         return yb, None, None, None, None
 
 

@@ -99,10 +99,13 @@ class Plan:
         k = (c_int * TUNING_KNOBS)(*[int(x) for x in knobs])
         check(_lib.load().aeolus_plan_set_tuning(self.handle, k))
 
-    def workspace(self, op: int, batch: int) -> torch.Tensor:
+    def workspace_bytes(self, op: int, batch: int) -> int:
         n = c_size_t()
         check(_lib.load().aeolus_workspace_bytes(self.handle, int(op), int(batch), byref(n)))
-        return torch.empty(n.value, dtype=torch.uint8, device=self.device)
+        return n.value
+
+    def workspace(self, op: int, batch: int) -> torch.Tensor:
+        return torch.empty(self.workspace_bytes(op, batch), dtype=torch.uint8, device=self.device)
 
     def close(self):
         if self.handle:
@@ -476,6 +479,42 @@ def swe_rk4_adjoint(plan_id: int, radius: float, omega: float, gravity: float, m
         prm = _swe_params(radius, omega, gravity, mean_depth, nu4, forcing, p.lmax, s.device)
         check(_lib.load().aeolus_swe_rk4_adjoint(p.handle, byref(prm), _ptr(s), _ptr(yb), B, float(dt), _ptr(w),
                                                  w.numel(), _stream(s.device)))
+    return yb.reshape(lead + (3,) + _spec_shape(p.lmax))
+
+
+def swe_rk4_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
+                   state: torch.Tensor, dt: float, forcing: torch.Tensor | None = None,
+                   step: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
+    """(step output or None without `step`, inputs of stages 2 to 4 as
+    [3, B, 3, L+1, L+1]) of one RK4 step from `state`."""
+    p = _PLANS[plan_id]
+    s, lead = _flat_spec(state, p.lmax, 3)
+    B = s.shape[0]
+    nxt = torch.empty_like(s) if step else None
+    stages = torch.empty((3,) + tuple(s.shape), dtype=s.dtype, device=s.device)
+    if B:
+        w = p.workspace(_lib.OP_SWE_RK4, B)
+        prm = _swe_params(radius, omega, gravity, mean_depth, nu4, forcing, p.lmax, s.device)
+        check(_lib.load().aeolus_swe_rk4_stages(p.handle, byref(prm), _ptr(s), _ptr(nxt) if step else None,
+                                                _ptr(stages), B, float(dt), _ptr(w), w.numel(), _stream(s.device)))
+    return nxt.reshape(lead + (3,) + _spec_shape(p.lmax)) if step else None, stages
+
+
+def swe_rk4_adjoint_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
+                           state: torch.Tensor, stages: torch.Tensor, state_bar: torch.Tensor, dt: float,
+                           forcing: torch.Tensor | None = None) -> torch.Tensor:
+    """swe_rk4_adjoint with the stage inputs of swe_rk4_stages."""
+    p = _PLANS[plan_id]
+    s, lead = _flat_spec(state, p.lmax, 3)
+    yb = _flat_spec(state_bar, p.lmax, 3)[0].clone()
+    B = s.shape[0]
+    if stages.shape != (3,) + tuple(s.shape) or stages.dtype != s.dtype or not stages.is_contiguous():
+        raise ValueError("swe_rk4_adjoint_stages needs the stages of swe_rk4_stages for this state")
+    if B:
+        w = p.workspace(_lib.OP_SWE_RK4_ADJOINT, B)
+        prm = _swe_params(radius, omega, gravity, mean_depth, nu4, forcing, p.lmax, s.device)
+        check(_lib.load().aeolus_swe_rk4_adjoint_stages(p.handle, byref(prm), _ptr(s), _ptr(stages), _ptr(yb), B,
+                                                        float(dt), _ptr(w), w.numel(), _stream(s.device)))
     return yb.reshape(lead + (3,) + _spec_shape(p.lmax))
 
 

@@ -476,6 +476,20 @@ int aeolus_swe_rk4_adjoint(aeolus_plan plan, const aeolus_swe_params* p,
                            const double* state, double* state_bar, int batch,
                            double dt, void* work, size_t work_bytes,
                            void* stream);
+/* One RK4 step out of place that keeps the inputs of stages 2, 3 and 4
+ * (stages: 3 states of the batch, one after the other).  next = the step's
+ * output, or NULL to stop after the third stage.  Workspace of
+ * AEOLUS_OP_SWE_RK4. */
+int aeolus_swe_rk4_stages(aeolus_plan plan, const aeolus_swe_params* p,
+                          const double* state, double* next, double* stages,
+                          int batch, double dt, void* work, size_t work_bytes,
+                          void* stream);
+/* aeolus_swe_rk4_adjoint with those stage inputs instead of recomputing
+ * them.  Workspace of AEOLUS_OP_SWE_RK4_ADJOINT. */
+int aeolus_swe_rk4_adjoint_stages(aeolus_plan plan, const aeolus_swe_params* p,
+                                  const double* state, const double* stages,
+                                  double* state_bar, int batch, double dt,
+                                  void* work, size_t work_bytes, void* stream);
 
 #ifdef __cplusplus
 }
