@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(TH128 ? kPfaThreads : 256, TH128 ? 7 : 3)
 }
 
 template <class Derive>
-__global__ void __launch_bounds__(256) g_slice_synth(Grouped<SliceSynthArg<Derive>> g) {
+__global__ void __launch_bounds__(kSynthSliceThreads, DeriveHasDf<Derive>::value ? 6 : 8) g_slice_synth(Grouped<SliceSynthArg<Derive>> g) {
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) g_slice_synth(Grouped<SliceSynthArg<Deriv
 }
 
 template <int NF>
-__global__ void __launch_bounds__(256) g_slice_anal(Grouped<SliceAnalArg> g) {
+__global__ void __launch_bounds__(kAnalSliceThreads, 8) g_slice_anal(Grouped<SliceAnalArg> g) {
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
@@ -477,7 +477,7 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
     return s;
   {
     ProfScope prof("ens_split_synth_slice", st);
-    launch_pdl(k1, dim3(gss.start[ng]), dim3(256), sm_ss, st, gss);
+    launch_pdl(k1, dim3(gss.start[ng]), dim3(kSynthSliceThreads), sm_ss, st, gss);
     AE_LAUNCH("g_slice_synth");
   }
   {
@@ -493,7 +493,7 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
   }
   {
     ProfScope prof("ens_split_anal_slice", st);
-    launch_pdl(k4, dim3(gsa.start[ng]), dim3(256), sm_sa, st, gsa);
+    launch_pdl(k4, dim3(gsa.start[ng]), dim3(kAnalSliceThreads), sm_sa, st, gsa);
     AE_LAUNCH("g_slice_anal");
   }
   ProfScope prof("ens_tc_anal_bf16x6", st);

@@ -158,8 +158,12 @@ __device__ __forceinline__ long long pk_pack(long long M, int e) {
 }
 
 // Packed word aligned to block exponent S >= its magnitude bound - 52:
-// rint(M 2^(e - S)).
-__device__ __forceinline__ long long pk_align(long long w, int S) { return fx_rshift(pk_mant(w), S - pk_exp(w)); }
+// rint(M 2^(e - S)) (half up): the mantissa and the shift taken in one, down to
+// one bit below the unit (shifts past 54 give 0, as does a clamped 63).
+__device__ __forceinline__ long long pk_align(long long w, int S) {
+  const int s = max(10, min(63, S - pk_exp(w) + 9));
+  return ((w >> s) + 1) >> 1;
+}
 
 // 2^p as a float in two factors (p1 + p2 = p, each a normal float).
 __device__ __forceinline__ float fx_pow2f(int p) { return __int_as_float((p + 127) << 23); }

@@ -101,25 +101,31 @@ struct DeriveHasDf : std::false_type {};
 template <class D>
 struct DeriveHasDf<D, std::enable_if_t<D::kColumnDf>> : std::true_type {};
 
-// One digit (|r| <= 128) as a bf16, exactly: the magic-number construction
-// puts r in the mantissa of 1.5 2^23 (FMA pipe, no integer-to-float
-// conversion, which would run on the FP64 pipe for 64-bit operands), and a
-// float holding a small integer is its own bf16 upper half.
-__device__ __forceinline__ __nv_bfloat16 digit_bf16(int r) {
-  const float f = __int_as_float(0x4B400000 + r) - 12582912.0f;
-  return __ushort_as_bfloat16(static_cast<unsigned short>(__float_as_uint(f) >> 16));
+// Balanced base-256 digits (-128..127; the first -128..128) of a fixed-point
+// integer X (|X| <= 2^47), most significant first, as floats.  Adding 128 to
+// every digit but the first makes them the bytes of X, with no carry to pass
+// on; a byte goes into the mantissa of 2^23 with one permute, and a float holding
+// a small integer is its own bf16 upper half.  Against one digit after the
+// other with 64-bit steps: analysis slicing 38.3 -> DIGA us and synthesis slicing
+// 97 -> DIGS us at 64 members, l_max 127.
+__device__ __forceinline__ void digit_floats(long long X, float* d) {
+  const long long Y = X + 0x8080808080ll;
+  const unsigned lo = static_cast<unsigned>(Y);
+  const int hi = static_cast<int>(Y >> 32);
+  const float bias = 8388736.0f;  // 2^23 + 128
+  d[5] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7650)) - bias;
+  d[4] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7651)) - bias;
+  d[3] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7652)) - bias;
+  d[2] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7653)) - bias;
+  d[1] = __uint_as_float(__byte_perm(static_cast<unsigned>(hi), 0x4B000000u, 0x7650)) - bias;
+  d[0] = __int_as_float(0x4B400000 + (hi >> 8)) - 12582912.0f;
 }
-
-// Balanced base-256 digits of a fixed-point integer X (|X| <= 2^47), most
-// significant first.
 __device__ inline void digits_from_fixed(long long X, __nv_bfloat16* d) {
+  static_assert(kSlices == 6, "48-bit values in six digits");
+  float f[kSlices];
+  digit_floats(X, f);
 #pragma unroll
-  for (int i = kSlices - 1; i >= 1; --i) {
-    const int r = static_cast<int>(((X + 128) & 255) - 128);
-    d[i] = digit_bf16(r);
-    X = (X - r) >> 8;
-  }
-  d[0] = digit_bf16(static_cast<int>(X));
+  for (int i = 0; i < kSlices; ++i) d[i] = __ushort_as_bfloat16(static_cast<unsigned short>(__float_as_uint(f[i]) >> 16));
 }
 
 // Balanced base-256 digits of rint(x 2^(48-E)), most significant first.
@@ -165,41 +171,41 @@ __device__ inline double scaled_to_double(long long T, int e) {
 // two exact steps.
 __device__ inline float pow2f(int p) { return __int_as_float((p + 127) << 23); }  // p in [-126, 127]
 
-__device__ inline df levels_to_df(const float* acc, int e) {
-  // pairwise: three exact two-sums of neighbouring levels, then two Dekker
-  // additions (error ~2^-48 of the operands) -- half the dependency depth of
-  // a sequential sum, for the latency-bound epilogue warps
-  const df p0 = two_sum(acc[0] * pow2f(40), acc[1] * pow2f(32));
-  const df p1 = two_sum(acc[2] * pow2f(24), acc[3] * pow2f(16));
-  const df p2 = two_sum(acc[4] * pow2f(8), acc[5]);
-  const df s = df_add_fast(df_add_fast(p0, p1), p2);
-  // s * 2^e, e = e1 + e2 with both factors normal floats
-  const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
-  return df{s.hi * pow2f(e1) * pow2f(e2), s.lo * pow2f(e1) * pow2f(e2)};
+// Two outputs at once on the packed two-lane pipe.  Pairwise: the three sums
+// of neighbouring levels, then two double-float additions (error ~2^-48 of the
+// operands), half the dependency depth of a sequential sum for the
+// latency-bound epilogue warps.  In every sum the first term is a multiple of
+// the second's last bit (integers below 2^24 eight bits apart, then sums of two
+// sixteen apart), so the three-step sum gives the exact error.
+__device__ inline df2 fast_scaled_sum2(f2 a, f2 p, f2 b) {  // a p + b
+  const f2 s = f2_fma(a, p, b);
+  return df2{s, f2_sub(b, f2_fma(a, f2_neg(p), s))};
 }
-
-// levels_to_df of two outputs at once (packed two-lane FP32; the same
-// operations, so the same results).
 __device__ inline void levels_to_df2(const float* a, const float* b, int ea, int eb, df& ra, df& rb) {
-  const f2 c40 = f2_splat(pow2f(40)), c32 = f2_splat(pow2f(32)), c24 = f2_splat(pow2f(24));
-  const f2 c16 = f2_splat(pow2f(16)), c8 = f2_splat(pow2f(8));
-  const df2 p0 = two_sum2(f2_mul(f2_pack(a[0], b[0]), c40), f2_mul(f2_pack(a[1], b[1]), c32));
-  const df2 p1 = two_sum2(f2_mul(f2_pack(a[2], b[2]), c24), f2_mul(f2_pack(a[3], b[3]), c16));
-  const df2 p2 = two_sum2(f2_mul(f2_pack(a[4], b[4]), c8), f2_pack(a[5], b[5]));
-  const df2 s = df2_add_fast(df2_add_fast(p0, p1), p2);
+  const f2 c8 = f2_splat(256.0f), c16 = f2_splat(65536.0f);
+  const df2 p0 = fast_scaled_sum2(f2_pack(a[0], b[0]), c8, f2_pack(a[1], b[1]));
+  const df2 p1 = fast_scaled_sum2(f2_pack(a[2], b[2]), c8, f2_pack(a[3], b[3]));
+  const df2 p2 = fast_scaled_sum2(f2_pack(a[4], b[4]), c8, f2_pack(a[5], b[5]));
+  df2 s = fast_scaled_sum2(p0.hi, c16, p1.hi);
+  s = fast_two_sum2(s.hi, f2_add(s.lo, f2_fma(p0.lo, c16, p1.lo)));
+  df2 t = fast_scaled_sum2(s.hi, c16, p2.hi);
+  t = fast_two_sum2(t.hi, f2_add(t.lo, f2_fma(s.lo, c16, p2.lo)));
   const int ea1 = max(-126, min(127, ea)), ea2 = max(-126, min(127, ea - ea1));
   const int eb1 = max(-126, min(127, eb)), eb2 = max(-126, min(127, eb - eb1));
   const f2 s1 = f2_pack(pow2f(ea1), pow2f(eb1)), s2 = f2_pack(pow2f(ea2), pow2f(eb2));
-  df2_unpack(df2{f2_mul(f2_mul(s.hi, s1), s2), f2_mul(f2_mul(s.lo, s1), s2)}, ra, rb);
+  df2_unpack(df2{f2_mul(f2_mul(t.hi, s1), s2), f2_mul(f2_mul(t.lo, s1), s2)}, ra, rb);
 }
 
 // Level recombination: T = sum_k I_k 256^(5-k), k = 0..5 <-> s+t = 2..7.
 // One K segment (<= 160 deep): |I_0| < 160 * 2^14, so |T| < 2^62.
 __device__ inline long long combine_levels(const float* acc) {
-  long long T = 0;
+  static_assert(kLevels == 6, "three pairs of levels");
+  int v[kLevels];
 #pragma unroll
-  for (int k = 0; k < kLevels; ++k) T = (T << 8) + __float2int_rn(acc[k]);
-  return T;
+  for (int k = 0; k < kLevels; ++k) v[k] = __float2int_rn(acc[k]);
+  // |I_k| <= (k + 1) 160 2^14: the first two pairs fit 32 bits
+  const long long U = fx_madw(v[0] * 256 + v[1], 1 << 16, v[2] * 256 + v[3]);
+  return fx_madw(v[4], 256, v[5]) + static_cast<long long>(static_cast<unsigned long long>(U) << 16);
 }
 
 // Exact-accumulation depth: the deepest level (6 digit pairs) sums at most
@@ -253,13 +259,12 @@ __device__ inline void store_digits8(__nv_bfloat16* tile, int r, int k0, const l
   uint32_t w[kSlices][4];
 #pragma unroll
   for (int u = 0; u < 8; u += 2) {
-    __nv_bfloat16 a[kSlices], b[kSlices];
-    digits_from_fixed(X[u], a);
-    digits_from_fixed(X[u + 1], b);
+    float a[kSlices], b[kSlices];
+    digit_floats(X[u], a);
+    digit_floats(X[u + 1], b);
 #pragma unroll
-    for (int s = 0; s < kSlices; ++s)
-      w[s][u >> 1] = static_cast<uint32_t>(__bfloat16_as_ushort(a[s])) |
-                     (static_cast<uint32_t>(__bfloat16_as_ushort(b[s])) << 16);
+    for (int s = 0; s < kSlices; ++s)  // the upper halves of both
+      w[s][u >> 1] = __byte_perm(__float_as_uint(a[s]), __float_as_uint(b[s]), 0x7632);
   }
   __nv_bfloat16* base = tile + tile_elem(kNT, 0, r, k0);
 #pragma unroll
@@ -350,8 +355,16 @@ __device__ __forceinline__ void split_synth_slice_body(const SplitDims& dm, cons
   }
 }
 
-// Four CTAs per SM (64 registers) for the FP64 derives; three (85) for the
-// double-float ones, whose packed columns spill at 64 registers.
+// 1,024 threads per SM (64 registers) for the FP64 derives; 768 (85) for the
+// double-float ones, whose packed columns spill at 64 registers.  Past one wave
+// the CTAs have 128 threads: the barriers between the three phases, which a
+// CTA's two members fill only in part, were the largest stall of 256 (3.6 of 11
+// cycles per issue); 92 -> 82 us at 64 members, l_max 127, but 6.5 -> 7.3 us with
+// one at l_max 85.
+constexpr int kSynthSliceThreads = 128;
+inline int synth_slice_threads(const aeolus_plan_impl* p, dim3 grid) {
+  return (long)grid.x * grid.y <= 4L * p->sm_count ? 256 : kSynthSliceThreads;
+}
 template <class Derive>
 __global__ void __launch_bounds__(256, DeriveHasDf<Derive>::value ? 3 : 4) split_synth_slice_kernel(SplitDims dm, const long long* __restrict__ kcum,
                                                                int batch, int mb, Derive der,
@@ -975,7 +988,7 @@ SplitParts split_synth_parts(const aeolus_plan_impl* p, int batch, void* scratch
   r.digits = reinterpret_cast<__nv_bfloat16*>(w);
   w += align256((size_t)p->split->h_kcum[r.dm.L + 1] * r.dm.ntiles * kSlices * kNT * 2);
   r.ecol = reinterpret_cast<int*>(w);
-  // 32 KB of staged values: four 256-thread CTAs per SM (64 registers each)
+  // 32 KB of staged values: six 128-thread CTAs per SM
   r.mb = slice_members(NF, r.dm.L + 2, p->tune_slice_mb, 32 * 1024);
   // fewer members per CTA while that leaves at most one wave (12.3 -> 8.4 us
   // for 4 members at l_max 85, 12.9 -> 8.2 for 16 at 42; past one wave it costs:
@@ -1016,7 +1029,7 @@ int launch_split_synth(const aeolus_plan_impl* p, const Derive& d, double2* FG, 
   if (s) return s;
   {
     ProfScope prof("split_synth_slice", st);
-    launch_pdl(k1, r.grid, dim3(256), r.smem, st, r.dm, p->split->kcum, batch, r.mb, d, r.digits, r.ecol);
+    launch_pdl(k1, r.grid, dim3(synth_slice_threads(p, r.grid)), r.smem, st, r.dm, p->split->kcum, batch, r.mb, d, r.digits, r.ecol);
     AE_LAUNCH("split_synth_slice_kernel");
   }
   const size_t sm2 = tc_smem_bytes();
