@@ -106,8 +106,8 @@ struct DeriveHasDf<D, std::enable_if_t<D::kColumnDf>> : std::true_type {};
 // every digit but the first makes them the bytes of X, with no carry to pass
 // on; a byte goes into the mantissa of 2^23 with one permute, and a float holding
 // a small integer is its own bf16 upper half.  Against one digit after the
-// other with 64-bit steps: analysis slicing 38.3 -> DIGA us and synthesis slicing
-// 97 -> DIGS us at 64 members, l_max 127.
+// other with 64-bit steps: analysis slicing 38 -> 30 us and, with the smaller CTAs
+// of split_synth_slice_kernel, synthesis slicing 97 -> 82 us at 64 members, l_max 127.
 __device__ __forceinline__ void digit_floats(long long X, float* d) {
   const long long Y = X + 0x8080808080ll;
   const unsigned lo = static_cast<unsigned>(Y);
