@@ -519,8 +519,11 @@ __device__ __forceinline__ void row_pfa_body(const RowArgs& a, const Pw& pw, con
   }
 }
 
+// Six CTAs per SM (80 registers); rows that start from the grid eight (64: 239
+// -> 217 us for 84 members of 6 fields at 192 x 384; chains are equal or slower
+// with seven or eight: gradient 13.34 -> 13.46 and 13.55 ms).
 template <class Pw, int IN_MODE, int OUT_MODE, class S, int T>
-__global__ void __launch_bounds__(T, T == kPfaThreads ? 6 : 2) row_kernel_pfa(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
+__global__ void __launch_bounds__(T, T != kPfaThreads ? 2 : IN_MODE == kInF ? 6 : 8) row_kernel_pfa(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                               FxConst kc) {
   pdl_wait();
   row_pfa_body<Pw, IN_MODE, OUT_MODE, S, T>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
