@@ -476,7 +476,7 @@ int swe_stages(const aeolus_plan_impl* plan, const aeolus_swe_params* p, const d
   const double2* in = state;
   for (int stage = 1; stage <= (step ? 4 : 3); ++stage) {
     SweDerive d{sp, in, fp, cor, 2.0 * p->omega};
-    Rk4 rk{stage, dt, y0, stage < 4 ? next[stage - 1] : nullptr, kacc, nullptr};
+    Rk4 rk = rk4_stage(stage, dt, y0, stage < 4 ? next[stage - 1] : nullptr, kacc);
     SweEpi e{sp, in, phi0, p->nu4, rk, spec_cor ? 2.0 * p->omega : 0.0, cor};
     e.forcing = reinterpret_cast<const double2*>(p->forcing);
     const int s = spec_cor ? run_full_chain(plan, SweDerive7{d}, pw, e, batch, chain, nullptr, st)
@@ -597,7 +597,7 @@ extern "C" int aeolus_bve_rk4_adjoint(aeolus_plan plan, const aeolus_bve_params*
   const double2* in = y0;
   for (int stage = 1; stage <= 3; ++stage) {
     BveDerive d{sp, in, f10};
-    Rk4 rk{stage, dt, y0, next[stage - 1], kacc, nullptr};
+    Rk4 rk = rk4_stage(stage, dt, y0, next[stage - 1], kacc);
     BveEpi e{sp, in, nullptr, p->viscosity, rk};
     if ((s = run_full_chain(plan, d, JacPw{}, e, batch, chain, nullptr, st))) return s;
     in = next[stage - 1];

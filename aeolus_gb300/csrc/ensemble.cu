@@ -265,7 +265,7 @@ struct BveModel {
     const double2* in = stage == 1 ? y0 : b.ystage;
     d = BveDerive{sp, in, 2.0 * E->prm[k].omega * kSqrt4PiOver3};
     pw = JacPw{};
-    e = BveEpi{sp, in, nullptr, E->prm[k].viscosity, Rk4{stage, dt, y0, b.ystage, b.acc, nullptr}};
+    e = BveEpi{sp, in, nullptr, E->prm[k].viscosity, rk4_stage(stage, dt, y0, b.ystage, b.acc)};
   }
 };
 
@@ -319,7 +319,7 @@ struct SweModel {
     double2* next = b.stage[(stage + 1) & 1];
     d = SweDerive{sp, in, fp, cor, 2.0 * q.omega};
     pw = SwePw{fp, phi0, (float)phi0};
-    e = SweEpi{sp, in, phi0, q.nu4, Rk4{stage, dt, y0, next, b.acc, nullptr}, spec_cor ? 2.0 * q.omega : 0.0, cor};
+    e = SweEpi{sp, in, phi0, q.nu4, rk4_stage(stage, dt, y0, next, b.acc), spec_cor ? 2.0 * q.omega : 0.0, cor};
     e.forcing = reinterpret_cast<const double2*>(q.forcing);
   }
 };

@@ -466,7 +466,7 @@ extern "C" int aeolus_bve_rk4(aeolus_plan plan, const aeolus_bve_params* p, doub
     for (int stage = 1; stage <= 4; ++stage) {
       const double2* in = stage == 1 ? y0 : ystage;
       BveDerive d{sp, in, f10};
-      Rk4 rk{stage, dt, y0, ystage, acc, nullptr};
+      Rk4 rk = rk4_stage(stage, dt, y0, ystage, acc);
       BveEpi e{sp, in, nullptr, p->viscosity, rk};
       if ((s = run_full_chain(plan, d, JacPw{}, e, batch, chain, nullptr, st))) return s;
     }
@@ -506,7 +506,7 @@ extern "C" int aeolus_swe_rk4(aeolus_plan plan, const aeolus_swe_params* p, doub
       const double2* in = stage == 1 ? y0 : stage_buf[stage & 1];        // 2 -> buf0, 3 -> buf1, 4 -> buf0
       double2* next = stage_buf[(stage + 1) & 1];                        // 1 -> buf0, 2 -> buf1, 3 -> buf0
       SweDerive d{sp, in, fp, cor, 2.0 * p->omega};
-      Rk4 rk{stage, dt, y0, next, acc, nullptr};
+      Rk4 rk = rk4_stage(stage, dt, y0, next, acc);
       SweEpi e{sp, in, phi0, p->nu4, rk, spec_cor ? 2.0 * p->omega : 0.0, cor};
       e.forcing = reinterpret_cast<const double2*>(p->forcing);
       s = spec_cor ? run_full_chain(plan, SweDerive7{d}, pw, e, batch, chain, status, st)

@@ -28,7 +28,7 @@ struct Spec {  // shared spectral context
   const double* xb;
   const double* dcoef;   // [(L+1)^2][8] combined SWE derive coefficients (plan radius only)
   const float2* dcoef_df;  // the same as double-floats (hi, lo), or none
-  __device__ double lap(int l) const { return -(double)l * (l + 1.0) * ir2; }
+  __device__ double lap(int l) const { return -(double)(l * (l + 1)) * ir2; }
   __device__ double2 at(const double2* a, int l, int m) const { return a[(long)l * (L + 1) + m]; }
   // Helmholtz inverse with l = 0 -> 0 (physics/barotropic.py:91); a
   // multiplication by the tabulated reciprocal (within 1 ulp of the divide).
@@ -174,7 +174,7 @@ struct JacPw {  // J = (a_snt b_lam - a_lam b_snt) / cos^2
 // modes 1..4: stage s of the classical RK4 (run/engine.py:406-431).
 struct Rk4 {
   int mode;
-  double dt;
+  double dt;        // times k in what is written: dt / 2, dt / 2, dt, dt / 6 (rk4_stage; 0 in mode 0)
   double2* y0;      // step-start state (updated at stage 4)
   double2* ystage;  // stage input for the next stage
   double2* acc;     // k1 + 2 k2 + 2 k3
@@ -196,15 +196,15 @@ struct Rk4 {
       tend[i] = k;
     } else if (mode == 1) {
       acc[i] = k;
-      ystage[i] = cadd(in.y, cscale(0.5 * dt, k));
+      ystage[i] = cadd(in.y, cscale(dt, k));
     } else if (mode == 2) {
       acc[i] = cadd(in.a, cscale(2.0, k));
-      ystage[i] = cadd(in.y, cscale(0.5 * dt, k));
+      ystage[i] = cadd(in.y, cscale(dt, k));
     } else if (mode == 3) {
       acc[i] = cadd(in.a, cscale(2.0, k));
       ystage[i] = cadd(in.y, cscale(dt, k));
     } else {
-      y0[i] = cadd(in.y, cscale(dt / 6.0, cadd(in.a, k)));
+      y0[i] = cadd(in.y, cscale(dt, cadd(in.a, k)));
     }
   }
   __device__ void zero(long i) const {
@@ -214,6 +214,12 @@ struct Rk4 {
     else y0[i] = z;
   }
 };
+
+// The divisions and products of the step are the host's: a division in every
+// thread of the last stage is ten multiply-adds of the FP64 pipe.
+inline Rk4 rk4_stage(int stage, double dt, double2* y0, double2* ystage, double2* acc) {
+  return Rk4{stage, stage == 4 ? dt / 6.0 : stage == 3 ? dt : 0.5 * dt, y0, ystage, acc, nullptr};
+}
 
 struct BveEpi {  // -trunc(A J) + nu lap zeta (+ forcing), l = 0 row zero
   static constexpr int NF = 1;
