@@ -703,18 +703,18 @@ def _rel_l2_fields(a, b):
 # workload: dram__bytes_read.sum + dram__bytes_write.sum from one ncu capture
 # of the first RK4 stage (cold L2).
 NCU_TRAFFIC = {
-    "split_synth_slice": 27.497728e6 + 86.54464e6,
-    "tc_synth_bf16x6": 138.119424e6 + 174.368e6,
-    "rows_fx_c2r_products_r2c": 226.578432e6 + 75.243008e6,
-    "split_anal_slice": 100.69504e6 + 95.401472e6,
-    "tc_anal_bf16x6": 230.352896e6 + 67.960576e6,
+    "split_synth_slice": 27.700736e6 + 63.557632e6,
+    "tc_synth_bf16x6": 136.809728e6 + 170.381312e6,
+    "rows_fx_c2r_products_r2c": 226.566912e6 + 46.115584e6,
+    "split_anal_slice": 66.86592e6 + 40.166144e6,
+    "tc_anal_bf16x6": 165.085696e6 + 34.807296e6,
 }
 
 
 # Warp instructions per launch of the same kernels (smsp__inst_executed.sum
 # of the same capture), for the instruction-issue roofline of the row stage.
 NCU_WARP_INSTRUCTIONS = {
-    "rows_fx_c2r_products_r2c": 294.58e6,
+    "rows_fx_c2r_products_r2c": 276.61e6,
 }
 SM_COUNT, ISSUE_PER_SM_CLK = 152, 4  # GB300: 4 schedulers per SM, one warp instruction each per clock
 
