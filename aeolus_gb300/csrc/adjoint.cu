@@ -490,8 +490,8 @@ int swe_stages(const aeolus_plan_impl* plan, const aeolus_swe_params* p, const d
     Rk4 rk = rk4_stage(stage, dt, y0, stage < 4 ? next[stage - 1] : nullptr, kacc);
     SweEpi e{sp, in, phi0, p->nu4, rk, spec_cor ? 2.0 * p->omega : 0.0, cor};
     e.forcing = reinterpret_cast<const double2*>(p->forcing);
-    const int s = spec_cor ? run_full_chain(plan, SweDerive7{d}, pw, e, batch, chain, nullptr, st)
-                           : run_full_chain(plan, d, pw, e, batch, chain, nullptr, st);
+    const int s = split_on(plan) ? run_full_chain(plan, SweDerive7{d}, pw, e, batch, chain, nullptr, st)
+                                 : run_full_chain(plan, d, pw, e, batch, chain, nullptr, st);
     if (s) return s;
     if (stage < 4) in = next[stage - 1];
   }
@@ -546,6 +546,8 @@ extern "C" int aeolus_swe_rk4_stages(aeolus_plan plan, const aeolus_swe_params* 
   int s = check_common(plan, "aeolus_swe_rk4_stages", batch, state, stages);
   if (s || (s = swe_check(p, "aeolus_swe_rk4_stages")) || batch == 0) return s;
   if (!std::isfinite(dt)) return fail(AEOLUS_ERR_ARG, "aeolus_swe_rk4_stages: dt must be finite");
+  if (plan->precision == AEOLUS_PREC_SPLIT_BF16 && !split_on(plan))  // as aeolus_swe_rk4
+    return fail(AEOLUS_ERR_ARG, "derived-field synthesis needs a split-precision Gauss plan");
   if (state == next || state == stages || next == stages)
     return fail(AEOLUS_ERR_ARG, "aeolus_swe_rk4_stages: arrays alias");
   const size_t sb = align256(state_bytes(plan, 3, batch));
