@@ -10,7 +10,7 @@ import torch
 import aeolus_gb300 as ae
 from aeolus_gb300 import _lib, adjoint, workloads as W
 from aeolus_gb300.adjoint import swe_rk4_checkpointed
-from aeolus_gb300.ops import _swe_params, swe_rk4_adjoint, swe_rk4_adjoint_stages, swe_rk4_stages
+from aeolus_gb300.ops import _swe_params, swe_rk4, swe_rk4_adjoint, swe_rk4_adjoint_stages, swe_rk4_stages
 from aeolus_gb300.shallow_water import ShallowWaterModel
 
 pytestmark = pytest.mark.gpu
@@ -74,3 +74,22 @@ def test_argument_errors():
     assert call(ok[0], ok[0], ok[2], w.numel()) == _lib.ERR_ARG
     assert call(ok[0], ok[1], None, w.numel()) == _lib.ERR_ARG
     torch.cuda.synchronize()
+
+
+def test_split_point_sets():
+    """The step refuses a split point-set plan and so do kept stages; the step
+    adjoint takes one."""
+    from test_gpu_adjoint import points_plan
+
+    p = points_plan(8)
+    p.set_precision(_lib.PREC_SPLIT_BF16)
+    s0, depth = W.member_states(8, 2, seed=9)
+    y = torch.as_tensor(s0, device="cuda")
+    args = (p.id, W.EARTH_RADIUS, W.EARTH_OMEGA, W.GRAVITY, depth, 0.0)
+    with pytest.raises(ValueError):
+        swe_rk4(*args, y, 60.0, 1)
+    with pytest.raises(ValueError):
+        swe_rk4_stages(*args, y, 60.0)
+    g = swe_rk4_adjoint(*args, y, torch.ones_like(y).tril(), 60.0)
+    assert torch.isfinite(torch.view_as_real(g)).all() and g.abs().max() > 0
+    p.close()
