@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) g_legendre_analysis(Grouped<AnalArg<Epi>>
 }
 
 template <class Pw>
-__global__ void __launch_bounds__(kWideMaxThreads, 1) g_rows(Grouped<RowArg<Pw>> g, FxConst kc) {
+__global__ void __launch_bounds__(kWideMaxThreads, 2) g_rows(Grouped<RowArg<Pw>> g, FxConst kc) {
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];

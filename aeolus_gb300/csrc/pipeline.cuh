@@ -264,8 +264,8 @@ WideRowCfg wide_row_cfg(const aeolus_plan_impl* p, int batch) {
     }
     c.smem = row_w_smem_bytes<Pw>(f, c.nr);
     // few rows: twice the threads shorten each row; otherwise more CTAs per SM
-    if ((long)c.grid.x * c.grid.y <= 1L * p->sm_count) c.threads = 512;
-    else if ((long)c.grid.x * c.grid.y <= 2L * p->sm_count) c.threads = 256;
+    // (512 threads measured equal at one CTA per SM and 22 % slower at two)
+    if ((long)c.grid.x * c.grid.y <= 2L * p->sm_count) c.threads = 256;
   } else {
     c.gf = row_w_dft_group<Pw>(f, p->lmax);
     c.gtab = row_w_dft_smem<Pw>(f, p->lmax, c.gf, false) > 220 * 1024;
@@ -273,7 +273,7 @@ WideRowCfg wide_row_cfg(const aeolus_plan_impl* p, int batch) {
     const int items = (std::min(c.gf, Pw::NIN) + dft_fields<Pw::NIN>() - 1) / dft_fields<Pw::NIN>() * (f.N / 2 + 1);
     c.threads = 32 * leg_warps((items + 31) / 32);
   }
-  if (p->tune_row_threads > 0) c.threads = std::min(p->tune_row_threads, 256);
+  if (p->tune_row_threads > 0) c.threads = std::min(p->tune_row_threads, kWideMaxThreads);
   return c;
 }
 

@@ -214,7 +214,7 @@ constexpr int w_rows_per_cta() {
   constexpr int NF = Pw::NIN > Pw::NOUT ? Pw::NIN : Pw::NOUT;
   return NF >= 5 ? 1 : NF >= 3 ? 2 : NF == 2 ? 4 : 8;
 }
-constexpr int kWideMaxThreads = 512;
+constexpr int kWideMaxThreads = 256;
 
 // Where the row stage of an FP64 plan finds input field f of a functor:
 // spectra block src(f), times i m / R for a longitude derivative (lam(f)),
@@ -607,13 +607,13 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
 
 // ---------------------------------------------------------------- kernels
 template <class Pw, int NR, int IN_MODE, int OUT_MODE>
-__global__ void __launch_bounds__(kWideMaxThreads, 1) row_kernel_w(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
+__global__ void __launch_bounds__(kWideMaxThreads, 2) row_kernel_w(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                    FxConst kc) {
   pdl_wait();
   row_w_body<Pw, NR, IN_MODE, OUT_MODE>(a, pw, twfx, kc, blockIdx.x, blockIdx.y);
 }
 template <class Pw, int IN_MODE, int OUT_MODE, bool GTAB>
-__global__ void __launch_bounds__(kWideMaxThreads, 1) row_kernel_w_dft(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
+__global__ void __launch_bounds__(kWideMaxThreads, 2) row_kernel_w_dft(RowArgs a, Pw pw, const FxW* __restrict__ twfx,
                                                                        int gf) {
   pdl_wait();
   row_w_dft_body<Pw, IN_MODE, OUT_MODE, GTAB>(a, pw, twfx, gf, blockIdx.x, blockIdx.y);
