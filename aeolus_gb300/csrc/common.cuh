@@ -120,6 +120,10 @@ constexpr int kLegLow = 30, kLegBits = 59, kLegTerms = 16, kLegDrop = 8;
 __host__ __device__ inline long tri_off(int m, int L) { return (long)m * (L + 1) - (long)m * (m - 1) / 2; }
 __host__ __device__ inline long n_coeff(int L) { return (long)(L + 1) * (L + 2) / 2; }
 
+// Static shared memory (per-CTA scalars) of any kernel with dynamic shared memory
+// is below this; checked where a limit is raised (allow_smem_raw).
+constexpr size_t kStaticSmemMax = 4 * 1024;
+
 constexpr int kMaxFactors = 16;
 
 struct FftInfo {

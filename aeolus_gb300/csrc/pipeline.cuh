@@ -19,9 +19,12 @@ namespace aeolus {
 // into a CUDA graph -- do not touch the function attributes again.
 int allow_smem_raw(const void* kern, size_t bytes);  // plan.cu
 
+// A kernel's static shared memory counts towards both limits (48 KB without the
+// attribute, 227 KB with it): sizes that leave kStaticSmemMax of room need no look
+// at the kernel.
 template <class K>
 inline int allow_smem(K kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return AEOLUS_OK;
+  if (bytes + kStaticSmemMax <= 48 * 1024) return AEOLUS_OK;
   if (bytes > 227 * 1024) return fail(AEOLUS_ERR_ARG, "shared-memory tile exceeds 227 KB for this size");
   return allow_smem_raw(reinterpret_cast<const void*>(kern), bytes);
 }

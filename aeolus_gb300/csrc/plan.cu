@@ -425,6 +425,12 @@ int allow_smem_raw(const void* kern, size_t bytes) {
   std::lock_guard<std::mutex> g(mu);
   size_t& have = done[{kern, dev}];
   if (have >= bytes) return AEOLUS_OK;
+  cudaFuncAttributes attr;
+  AE_CUDA(cudaFuncGetAttributes(&attr, kern));
+  if (attr.sharedSizeBytes > kStaticSmemMax)
+    return fail(AEOLUS_ERR_CUDA, "a kernel's static shared memory exceeds kStaticSmemMax");
+  if (bytes + attr.sharedSizeBytes > 227 * 1024)
+    return fail(AEOLUS_ERR_ARG, "shared-memory tile exceeds 227 KB for this size");
   AE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   have = bytes;
   return AEOLUS_OK;
