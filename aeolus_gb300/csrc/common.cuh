@@ -111,12 +111,6 @@ __host__ __device__ inline long fg_index(long b, int m, int f, int j, int L, int
   return ((b * (L + 1) + m) * (long)nlat + j) * nblk + f;
 }
 
-// Fixed point of the FP64 plans' Legendre sums (legendre.cuh): factors below
-// 2^59 in limb pairs of 30 low bits (|high|, |low| <= 2^29, so the two mixed
-// products of 16 terms stay within 2^63), the sums kept less their last 8 bits
-// (2^80 a term: 2^14 terms).
-constexpr int kLegLow = 30, kLegBits = 59, kLegTerms = 16, kLegDrop = 8;
-
 __host__ __device__ inline long tri_off(int m, int L) { return (long)m * (L + 1) - (long)m * (m - 1) / 2; }
 __host__ __device__ inline long n_coeff(int L) { return (long)(L + 1) * (L + 2) / 2; }
 
@@ -164,11 +158,8 @@ struct aeolus_plan_impl {
   double* wq = nullptr;      // [nlat] w_gl * 2 pi / nlon
   double* coslat = nullptr;  // [nlat] or [npoints], max(cos lat, 1e-8)
   double* fgrid = nullptr;   // [nlat] or [npoints]: synthesis of the unit (1,0) mode
-  int2* P = nullptr;         // normalised P_lm in limb pairs (kLegBits), [tri_off(m)*nh + (l-m)*nh + jn] (row fastest)
-  int2* PT = nullptr;        // [tri_off(m)*nh + jn*(L+1-m) + (l-m)] (degree fastest)
-  int* eP = nullptr;         // [m][nh] exponents of P's (order, row) columns: P = limbs 2^(e - kLegBits)
-  int* ePT = nullptr;        // [tri_off(m) + (l-m)] exponents of PT's (order, degree) columns
-  double* sth = nullptr;     // [nlat] sin(colatitude)
+  double* P = nullptr;       // [tri_off(m)*nh + (l-m)*nh + jn]  (row jn fastest)
+  double* PT = nullptr;      // [tri_off(m)*nh + jn*(L+1-m) + (l-m)] (degree fastest)
   float4* twdf = nullptr;    // [nlon] the same twiddles as double-float (re.hi, re.lo, im.hi, im.lo)
   FxW* twfx = nullptr;       // [nlon] the same twiddles as Q61 31-bit limbs (fixed-point rows)
   int* fft_irev = nullptr;   // [fftx.n] position of natural index q in digit-reversed order (in-place FFTs)

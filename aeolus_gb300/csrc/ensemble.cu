@@ -61,7 +61,6 @@ template <class Derive>
 struct SynthArg {
   LegArgs a;
   Derive d;
-  int cpt;  // columns per thread
 };
 template <class Epi>
 struct AnalArg {
@@ -102,8 +101,7 @@ __global__ void __launch_bounds__(256) g_legendre_synth(Grouped<SynthArg<Derive>
   pdl_wait();
   const int k = g.find(blockIdx.x);
   const int loc = blockIdx.x - g.start[k];
-  if (g.arg[k].cpt == 2) legendre_synth_body<Derive, 2>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
-  else legendre_synth_body<Derive, 1>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
+  legendre_synth_body<Derive>(g.arg[k].a, g.arg[k].d, loc % g.gx[k], loc / g.gx[k]);
 }
 
 template <class Epi>
@@ -395,7 +393,7 @@ int ens_stage_m(const aeolus_ensemble_s* E, double2* const* y0, int stage, doubl
       const LegCfg cs = synth_cfg<SDerive>(p, E->batch[k]);
       const LegCfg ca = analysis_cfg<Epi>(p, E->batch[k]);
       grouped_add(gs, SynthArg<SDerive>{leg_args(p, cs, E->batch[k], FG, N64),
-                                        M::split_derive(der[k]), cs.cpt},
+                                        M::split_derive(der[k])},
                   cs.grid);
       grouped_add(ga, AnalArg<Epi>{leg_args(p, ca, E->batch[k], FG, N64), epi[k]},
                   ca.grid);

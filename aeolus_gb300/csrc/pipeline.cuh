@@ -14,6 +14,12 @@
 
 namespace aeolus {
 
+inline int pick_bc(int L, int batch) {
+  const long ctas = (long)n_pairs(L) * batch;
+  int bc = (int)std::max(1L, std::min(4L, ctas / 608));
+  return std::min(bc, std::max(batch, 1));
+}
+
 // Raises a kernel's dynamic shared-memory limit once per (kernel, device):
 // later calls -- including calls made while a stream is being captured
 // into a CUDA graph -- do not touch the function attributes again.
@@ -39,8 +45,7 @@ inline int round_threads(long items, int lo, int hi) {
 struct LegCfg {
   int bc;          // members per CTA
   int ss;          // CTAs per (order pair, member chunk)
-  int cpt, rb;     // synthesis: columns per thread, rows per warp
-  int js, solo;    // analysis
+  int solo;        // analysis: one order per CTA
   int threads;
   size_t smem;
   dim3 grid;
@@ -58,53 +63,45 @@ inline int leg_warps(int warps) {
 }
 
 // CTAs that share one (order pair, member chunk) of `warps` warps of items:
-// enough for four CTAs per SM (two: 10 % slower at one member, eight: equal at
-// eight members), none with fewer than four warps (each
-// repeats the derivation or the folding of the whole pair).
+// six CTAs per SM even out the last wave (8 members at l_max 127: 512 pairs
+// on 152 SMs are 4 rounds for 3.4 of work); no CTA gets fewer than two warps,
+// and its share of the columns' derivation stays a few percent.
 inline int leg_shares(const aeolus_plan_impl* p, long ctas, int warps) {
-  const long want = (4L * p->sm_count + ctas - 1) / std::max(ctas, 1L);
-  return (int)std::max(1L, std::min<long>(want, warps / 4));
+  const long want = (6L * p->sm_count + ctas - 1) / std::max(ctas, 1L);
+  return (int)std::max(1L, std::min<long>(want, warps / 2));
 }
 
 template <class Derive>
 LegCfg synth_cfg(const aeolus_plan_impl* p, int batch) {
   const int L = p->lmax;
-  int bc = p->tune_bc_synth > 0 ? std::min(p->tune_bc_synth, std::max(batch, 1)) : 1;
+  int bc = p->tune_bc_synth > 0 ? std::min(p->tune_bc_synth, std::max(batch, 1)) : pick_bc(L, batch);
   while (bc > 1 && synth_smem_bytes<Derive>(L, bc) > 200 * 1024) --bc;
-  const int gy = (batch + bc - 1) / bc, cols = bc * Derive::NF;
-  // two columns per thread share each basis value once there is a warp for
-  // every scheduler without it; rows per warp: the fewest warps (idle lanes are
-  // rows past the last one or slots past the last column), the widest of equals
-  const int cpt = cols > 1 && (long)n_pairs(L) * gy * p->nh * cols >= 2L * 32 * 8 * p->sm_count ? 2 : 1;
-  int rb = 32, warps = 0;
-  for (int r = 32; r >= 8; r /= 2) {
-    const int w = (p->nh + r - 1) / r * ((cols + 32 / r * cpt - 1) / (32 / r * cpt));
-    if (r == 32 || w < warps) rb = r, warps = w;
-  }
-  const int ss = leg_shares(p, (long)n_pairs(L) * gy, warps);
-  return LegCfg{bc, ss, cpt, rb, 1, 0, 32 * std::max(4, leg_warps((warps + ss - 1) / ss)), synth_smem_bytes<Derive>(L, bc),
-                dim3(n_pairs(L) * ss, gy)};
+  const int gy = (batch + bc - 1) / bc, items = p->nh * bc * Derive::NF;
+  const int ss = leg_shares(p, (long)n_pairs(L) * gy, (items + 31) / 32);
+  const int per = (items + ss - 1) / ss;
+  return LegCfg{bc, ss, 0, 32 * leg_warps((per + 31) / 32), synth_smem_bytes<Derive>(L, bc), dim3(n_pairs(L) * ss, gy)};
 }
 
 template <class Epi>
 LegCfg analysis_cfg(const aeolus_plan_impl* p, int batch) {
-  const int L = p->lmax, top = EpiTop<Epi>::top(L);
-  int bc = p->tune_bc_anal > 0 ? std::min(p->tune_bc_anal, std::max(batch, 1)) : 1;
-  while (bc > 1 && analysis_smem_bytes<Epi>(p->nh, bc, 0) > 160 * 1024) --bc;
-  const int solo = analysis_smem_bytes<Epi>(p->nh, bc, 0) > 227 * 1024;
-  const long pairs = solo ? top + 1 : n_pairs(top);
-  const int gy = (batch + bc - 1) / bc, degrees = bc * (top + 2);
-  // row slices: at most 128 rows per lane, and enough lanes for eight warps per SM
-  int js = 1;
-  while (js < 32 && (p->nh > js * 128 || (js < 8 && pairs * gy * degrees * js < 256L * p->sm_count))) js *= 2;
-  const int ss = leg_shares(p, pairs * gy, (degrees * js + 31) / 32);
-  const int per = (degrees + ss - 1) / ss;
-  return LegCfg{bc, ss, 1, 32, js, solo, 32 * std::max(4, leg_warps((per * js + 31) / 32)),
-                analysis_smem_bytes<Epi>(p->nh, bc, solo), dim3((unsigned)(pairs * ss), gy)};
+  const int L = p->lmax, top = EpiTop<Epi>::top(L), js = leg_row_slices(p->nh, Epi::NF);
+  int bc = p->tune_bc_anal > 0 ? std::min(p->tune_bc_anal, std::max(batch, 1)) : pick_bc(top, batch);
+  while (bc > 1 && analysis_smem_bytes<Epi>(L, p->nh, bc, 1, 0) > 160 * 1024) --bc;
+  const int solo = analysis_smem_bytes<Epi>(L, p->nh, bc, top + 2, 0) > 227 * 1024;
+  const int pairs = solo ? top + 1 : n_pairs(top);
+  const int gy = (batch + bc - 1) / bc, degrees = bc * (top + 2), q = 32 / js;  // q degrees fill a warp
+  const int want = leg_shares(p, (long)pairs * gy, (degrees * js + 31) / 32);
+  int per = (degrees + want - 1) / want;
+  per = std::max(std::min(q, degrees), per / q * q);
+  int ss = (degrees + per - 1) / per;
+  while (js > 1 && ss < degrees && analysis_smem_bytes<Epi>(L, p->nh, bc, ss, solo) > 220 * 1024) ++ss;  // partial sums that fit
+  per = (degrees + ss - 1) / ss;
+  return LegCfg{bc, ss, solo, std::max(128, 32 * leg_warps((per * js + 31) / 32)),
+                analysis_smem_bytes<Epi>(L, p->nh, bc, ss, solo), dim3(pairs * ss, gy)};
 }
 
 inline LegArgs leg_args(const aeolus_plan_impl* p, const LegCfg& c, int batch, double2* FG, int nblk) {
-  return LegArgs{p->lmax, p->nlat, p->nh, batch, c.bc, c.ss, c.rb, c.js, c.solo, p->P, p->eP, p->PT, p->ePT, FG, nblk};
+  return LegArgs{p->lmax, p->nlat, p->nh, batch, c.bc, c.ss, c.solo, p->P, p->PT, FG, nblk};
 }
 
 inline int row_threads(const aeolus_plan_impl* p) { return p->tune_row_threads > 0 ? p->tune_row_threads : 256; }
@@ -114,7 +111,7 @@ int launch_synth(const aeolus_plan_impl* p, const Derive& d, double2* FG, int nb
                  cudaStream_t st) {
   const LegCfg c = synth_cfg<Derive>(p, batch);
   const LegArgs a = leg_args(p, c, batch, FG, nblk);
-  auto kern = c.cpt == 2 ? legendre_synth_kernel<Derive, 2> : legendre_synth_kernel<Derive, 1>;
+  auto kern = legendre_synth_kernel<Derive>;
   int s = allow_smem(kern, c.smem);
   if (s) return s;
   ProfScope prof("legendre_synth_f64", st);

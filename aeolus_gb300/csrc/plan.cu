@@ -10,7 +10,6 @@
 
 #include "common.cuh"
 #include "fx.cuh"
-#include "w96.cuh"
 
 namespace aeolus {
 
@@ -186,15 +185,15 @@ __global__ void __launch_bounds__(kTabThreads) legendre_table_kernel(int L, int 
   const long base = tri_off(m, L) * nh;
   const int K = L + 1 - m;
   double* prow = P + base;
-  double* pcol = PT ? PT + base + (long)jn * K : nullptr;
+  double* pcol = PT + base + (long)jn * K;
   double p2 = pmm;
   double p1 = sqrt(2.0 * m + 3.0) * xv * pmm;
   if (on) {
     prow[jn] = pmm;
-    if (pcol) pcol[0] = pmm;
+    pcol[0] = pmm;
     if (m < L) {
       prow[(long)nh + jn] = p1;
-      if (pcol) pcol[1] = p1;
+      pcol[1] = p1;
     }
   }
   for (int l0 = m + 2; l0 <= L; l0 += kTabChunk) {
@@ -210,36 +209,12 @@ __global__ void __launch_bounds__(kTabThreads) legendre_table_kernel(int L, int 
       const double p = ca[i] * (xv * p1 - cb[i] * p2);
       if (on) {
         prow[(long)(l0 + i - m) * nh + jn] = p;
-        if (pcol) pcol[l0 + i - m] = p;
+        pcol[l0 + i - m] = p;
       }
       p2 = p1;
       p1 = p;
     }
   }
-}
-
-// FP64 table columns of `n` values (stride `inc`) to limb pairs in place, at one
-// exponent per column.
-__device__ void limbs_in_place(double* v, int n, long inc, int* e) {
-  unsigned key = 0u;
-#pragma unroll 8
-  for (int t = 0; t < n; ++t) key = max(key, f64_key(v[t * inc]));
-  const int E = f64_key_exp(key);
-  *e = E;
-  for (int t0 = 0; t0 < n; t0 += 8) {  // eight loads in flight
-    double x[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = t0 + u < n ? v[(t0 + u) * inc] : 0.0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (t0 + u < n) *reinterpret_cast<int2*>(v + (t0 + u) * inc) = limbs<kLegLow>(i64_of_f64_rn(x[u], E - kLegBits));
-  }
-}
-// P: one column per (order, row); PT: one per (order, degree) (grid.z = 1).
-__global__ void legendre_limbs_kernel(int L, int nh, double* P, int* eP, double* PT, int* ePT) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y, K = L + 1 - m;
-  if (blockIdx.z == 0 && i < nh) limbs_in_place(P + tri_off(m, L) * nh + i, K, nh, eP + (long)m * nh + i);
-  if (blockIdx.z == 1 && i < K) limbs_in_place(PT + tri_off(m, L) * nh + i, nh, K, ePT + tri_off(m, L) + i);
 }
 
 // coslat (clamped like spherical_backend.py:72,129) and the synthesis of
@@ -388,28 +363,12 @@ int common_tables(aeolus_plan_impl* p) {
   return AEOLUS_OK;
 }
 
-}  // namespace
-
-// The FP64 table in P's layout (the basis digits of a split-precision plan are
-// cut from it).
-int legendre_table_f64(const aeolus_plan_impl* p, double* P) {
-  legendre_table_kernel<<<dim3((p->nh + kTabThreads - 1) / kTabThreads, p->lmax + 1), kTabThreads>>>(p->lmax, p->nh, p->x, p->sth, P, nullptr);
-  AE_LAUNCH("legendre_table_kernel");
-  return AEOLUS_OK;
-}
-
-namespace {
-
 void free_plan(aeolus_plan_impl* p) {
-  double* bufs[] = {p->x, p->wq, p->coslat, p->fgrid, p->sth, p->basis, p->wpts,
+  double* bufs[] = {p->x, p->wq, p->coslat, p->fgrid, p->P, p->PT, p->basis, p->wpts,
                     p->latp, p->cplus, p->cminus, p->cplus_true, p->invlap, p->xa, p->xb, p->dcoef};
   for (double* b : bufs)
     if (b) cudaFree(b);
   if (p->dcoef_df) cudaFree(p->dcoef_df);
-  if (p->P) cudaFree(p->P);
-  if (p->PT) cudaFree(p->PT);
-  if (p->eP) cudaFree(p->eP);
-  if (p->ePT) cudaFree(p->ePT);
   if (p->twdf) cudaFree(p->twdf);
   if (p->twfx) cudaFree(p->twfx);
   if (p->fft_irev) cudaFree(p->fft_irev);
@@ -530,8 +489,8 @@ extern "C" int aeolus_plan_create_gauss(int nlat, int nlon, int lmax, double rad
   struct Tmp {  // node temporaries, freed on every exit path
     double* p = nullptr;
     ~Tmp() { if (p) cudaFree(p); }
-  } t_w, t_t;
-  double *&wgl = t_w.p, *&sth = p->sth, *&theta = t_t.p;
+  } t_w, t_s, t_t;
+  double *&wgl = t_w.p, *&sth = t_s.p, *&theta = t_t.p;
   if ((s = cuda_check(cudaMalloc(&p->x, nlat * sizeof(double)), "cudaMalloc"))) return bail(s);
   if ((s = cuda_check(cudaMalloc(&wgl, nlat * sizeof(double)), "cudaMalloc"))) return bail(s);
   if ((s = cuda_check(cudaMalloc(&sth, nlat * sizeof(double)), "cudaMalloc"))) return bail(s);
@@ -554,15 +513,10 @@ extern "C" int aeolus_plan_create_gauss(int nlat, int nlon, int lmax, double rad
   if ((s = cuda_check(cudaMalloc(&p->fgrid, nlat * sizeof(double)), "cudaMalloc"))) return bail(s);
   row_metrics_kernel<<<(nlat + 127) / 128, 128>>>(nlat, p->x, sth, p->coslat, p->fgrid);
   if ((s = cuda_check(cudaGetLastError(), "row_metrics_kernel"))) return bail(s);
-  if ((s = cuda_check(cudaMalloc(&p->P, ntab * sizeof(int2)), "cudaMalloc P"))) return bail(s);
-  if ((s = cuda_check(cudaMalloc(&p->PT, ntab * sizeof(int2)), "cudaMalloc PT"))) return bail(s);
-  if ((s = cuda_check(cudaMalloc(&p->eP, (size_t)(L + 1) * nh * sizeof(int)), "cudaMalloc eP"))) return bail(s);
-  if ((s = cuda_check(cudaMalloc(&p->ePT, n_coeff(L) * sizeof(int)), "cudaMalloc ePT"))) return bail(s);
-  double *P64 = reinterpret_cast<double*>(p->P), *PT64 = reinterpret_cast<double*>(p->PT);
-  legendre_table_kernel<<<dim3((nh + kTabThreads - 1) / kTabThreads, L + 1), kTabThreads>>>(L, nh, p->x, sth, P64, PT64);
+  if ((s = cuda_check(cudaMalloc(&p->P, ntab * sizeof(double)), "cudaMalloc P"))) return bail(s);
+  if ((s = cuda_check(cudaMalloc(&p->PT, ntab * sizeof(double)), "cudaMalloc PT"))) return bail(s);
+  legendre_table_kernel<<<dim3((nh + kTabThreads - 1) / kTabThreads, L + 1), kTabThreads>>>(L, nh, p->x, sth, p->P, p->PT);
   if ((s = cuda_check(cudaGetLastError(), "legendre_table_kernel"))) return bail(s);
-  legendre_limbs_kernel<<<dim3((std::max(nh, L + 1) + 63) / 64, L + 1, 2), 64>>>(L, nh, P64, p->eP, PT64, p->ePT);
-  if ((s = cuda_check(cudaGetLastError(), "legendre_limbs_kernel"))) return bail(s);
   std::vector<double2> tw;
   twiddles(nlon, tw);
   {

@@ -196,8 +196,6 @@ int split_build_points(aeolus_plan_impl* p) {
 
 }  // namespace
 
-int legendre_table_f64(const aeolus_plan_impl* p, double* P);  // plan.cu
-
 int split_build(aeolus_plan_impl* p) {
   if (p->split) return AEOLUS_OK;
   if (p->kind == kPoints) return split_build_points(p);
@@ -223,17 +221,10 @@ int split_build(aeolus_plan_impl* p) {
   AE_CUDA(cudaMalloc(&t->eana, (size_t)ana_row_tiles(L) * 128 * sizeof(int)));
   AE_CUDA(cudaMalloc(&t->err, sizeof(int)));
   AE_CUDA(cudaMemset(t->err, 0, sizeof(int)));
-  struct Table {  // FP64 basis, freed on every exit path
-    double* P = nullptr;
-    ~Table() { if (P) cudaFree(P); }
-  } tab;
-  AE_CUDA(cudaMalloc(&tab.P, n_coeff(L) * p->nh * sizeof(double)));
-  const int s = legendre_table_f64(p, tab.P);
-  if (s) return s;
-  split_psyn_kernel<<<dim3((t->Mt * 128 + 127) / 128, L + 1), 128>>>(L, p->nlat, p->nh, t->Mt, tab.P, t->kcum, t->psyn,
+  split_psyn_kernel<<<dim3((t->Mt * 128 + 127) / 128, L + 1), 128>>>(L, p->nlat, p->nh, t->Mt, p->P, t->kcum, t->psyn,
                                                                       t->esyn);
   AE_LAUNCH("split_psyn_kernel");
-  split_pana_kernel<<<dim3(1, ana_row_tiles(L)), 128>>>(L, p->nlat, p->nh, t->NK, tab.P, t->pana, t->eana);
+  split_pana_kernel<<<dim3(1, ana_row_tiles(L)), 128>>>(L, p->nlat, p->nh, t->NK, p->P, t->pana, t->eana);
   AE_LAUNCH("split_pana_kernel");
   AE_CUDA(cudaDeviceSynchronize());
   return AEOLUS_OK;
