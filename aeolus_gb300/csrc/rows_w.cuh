@@ -21,7 +21,7 @@
 //
 // Row lengths without a 2/3/5 transform (the 3/2-rule grids of state grids
 // that just resolve l_max: 3 l_max + 1 points) use a direct sum, folded about
-// the middle of the row, over 28-bit limb pairs with 64-bit accumulators:
+// the middle of the row, over 30-bit limb pairs with 64-bit accumulators:
 // six wide multiply-adds per order and pair of points (row_w_dft_body).
 //
 // Row stage per RK4 stage against FP64 transforms and sums: 8 members at 192 x
@@ -401,21 +401,31 @@ __device__ __forceinline__ void row_w_body(const RowArgs& a, const Pw& pw, const
 }
 
 // ------------------------------------------------------------ direct sums
-constexpr int kDftLow = 28, kDftBits = 55;  // |data|, |twiddle| < 2^55 in limb pairs of 28 low bits
-constexpr int kDftTerms = 128;              // products per 64-bit accumulator (below 2^62), then flushed
+// |data|, |twiddle| <= 2^59 in limb pairs of 30 low bits (|high|, |low| <= 2^29).
+// A term's two mixed products add up to at most 2^59, so 16 terms stay within
+// 64 bits; the flushed sums drop their last 10 bits (2^78 a term: 2^14 terms and
+// the factor 4 of both signs and both halves).
+// Rounded so, the data carry 2^-60 of their row's largest value and the products
+// dropped (low x low) are as small, against the 2^-53 to which an FP64 sum of
+// the row rounds; 55 bits and truncation raised the error of fields with steep
+// spectra by a quarter over FP64 sums.
+constexpr int kDftLow = 30, kDftBits = 59, kDftTerms = 16, kDftDrop = 10;
+constexpr int kDftUnit = kDftBits - kDftLow - kDftDrop;  // sums are in 2^-kDftUnit of the data's unit
 
-// Twiddle q (cos, -sin of 2 pi q / N) in 28-bit limbs of Q55, from the shared
+// Twiddle q (cos, -sin of 2 pi q / N) in limb pairs of Q59, from the shared
 // table or (rows too long for one) from the plan's Q61 table.
 template <bool GTAB>
 __device__ __forceinline__ int4 dft_twiddle(const int4* tab, const FxW* __restrict__ twfx, int q) {
   if constexpr (!GTAB) return tab[q];
   const FxW w = fx_ldw(&twfx[q]);
-  const int2 c = limbs<kDftLow>((((long long)w.ch << 31) + w.cl + 32) >> 6), s = limbs<kDftLow>((((long long)w.sh << 31) + w.sl + 32) >> 6);
+  constexpr int cut = 61 - kDftBits;
+  auto q59 = [](int h, int l) { return limbs<kDftLow>((((long long)h << 31) + l + (1 << (cut - 1))) >> cut); };
+  const int2 c = q59(w.ch, w.cl), s = q59(w.sh, w.sl);
   return make_int4(c.x, c.y, s.x, s.y);
 }
 
 // (sum_j a_j cos, sum_j b_j (-sin)) of angle 2 pi i j / N, j = 1..J, for FT
-// fields: units of 2^-27 of the data's unit.
+// fields: in units of 2^-kDftUnit of the data's unit.
 template <int FT, bool GTAB>
 __device__ __forceinline__ void dft_sums(const int4* __restrict__ d, int ld, int J, int i, int N, const int4* tab,
                                          const FxW* __restrict__ twfx, w96* C, w96* S) {
@@ -444,8 +454,8 @@ __device__ __forceinline__ void dft_sums(const int4* __restrict__ d, int ld, int
     }
 #pragma unroll
     for (int f = 0; f < FT; ++f) {
-      C[f] = w_add(C[f], limb_total<kDftLow>(chh[f], cx[f]));
-      S[f] = w_add(S[f], limb_total<kDftLow>(shh[f], sx[f]));
+      C[f] = w_add(C[f], limb_total<kDftLow, kDftDrop>(chh[f], cx[f]));
+      S[f] = w_add(S[f], limb_total<kDftLow, kDftDrop>(shh[f], sx[f]));
     }
   }
 }
@@ -496,8 +506,7 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
       if (mx) atomicMax(&sc.key[f], mx);
     }
     __syncthreads();
-    constexpr int fb = kDftBits;
-    if (tid < NIN) sc.S[tid] = f64_key_exp(sc.key[tid]) - fb;
+    if (tid < NIN) sc.S[tid] = f64_key_exp(sc.key[tid]) - kDftBits;
     __syncthreads();
     constexpr int FT = dft_fields<NIN>();
     for (int g0 = 0; g0 < NIN; g0 += gf) {
@@ -505,7 +514,7 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
       for (int idx = tid; idx < ng * (L + 1); idx += T) {
         const int q = idx / ng, f = idx - q * ng;
         const double2 v = load(g0 + f, q);
-        const int2 re = limbs<kDftLow>(i64_of_f64(v.x, sc.S[g0 + f])), im = limbs<kDftLow>(i64_of_f64(v.y, sc.S[g0 + f]));
+        const int2 re = limbs<kDftLow>(i64_of_f64_rn(v.x, sc.S[g0 + f])), im = limbs<kDftLow>(i64_of_f64_rn(v.y, sc.S[g0 + f]));
         data[f * ld + q] = make_int4(re.x, re.y, im.x, im.y);
       }
       __syncthreads();
@@ -517,10 +526,10 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
         dft_sums<FT, GTAB>(d, ld, L, k, N, tab, twfx, C, S);
 #pragma unroll
         for (int u = 0; u < FT; ++u) {
-          const int f = g0 + s * FT + u, e = sc.S[f] - (kDftBits - kDftLow);
+          const int f = g0 + s * FT + u, e = sc.S[f] - kDftUnit;
           const bool bad = sc.key[f] >= kNonFinite;
           const int4 v0 = d[u * ld];
-          const w96 V0 = w_shl64(((long long)v0.x << kDftLow) + v0.y, kDftBits - kDftLow);
+          const w96 V0 = w_shl64(((long long)v0.x << kDftLow) + v0.y, kDftUnit);
           const w96 p = w_add(C[u], S[u]), r = w_sub(C[u], S[u]);
           grid[f * N + k] = bad ? nan : f64_of_w(w_add(V0, w_add(p, p)), e);
           if (k > 0 && N - k > k) grid[f * N + N - k] = bad ? nan : f64_of_w(w_add(V0, w_add(r, r)), e);
@@ -571,15 +580,15 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
       for (int idx = tid; idx < ng * (J + 1); idx += T) {
         const int f = idx / (J + 1), i = idx - f * (J + 1), S = sc.S[g0 + f];
         const double* x = grid + (g0 + f) * N;
-        const long long X = i64_of_f64(x[i], S);
+        const long long X = i64_of_f64_rn(x[i], S);
         int2 p, r;
         if (i > 0) {
-          const long long Y = i64_of_f64(x[N - i], S);
+          const long long Y = i64_of_f64_rn(x[N - i], S);
           p = limbs<kDftLow>(X + Y);
           r = limbs<kDftLow>(X - Y);
         } else {  // x_0 and, for an even row, the point opposite
           p = limbs<kDftLow>(X);
-          r = limbs<kDftLow>(N % 2 == 0 ? i64_of_f64(x[half], S) : 0LL);
+          r = limbs<kDftLow>(N % 2 == 0 ? i64_of_f64_rn(x[half], S) : 0LL);
         }
         data[f * ld + i] = make_int4(p.x, p.y, r.x, r.y);
       }
@@ -591,10 +600,10 @@ __device__ __forceinline__ void row_w_dft_body(const RowArgs& a, const Pw& pw, c
         dft_sums<FT, GTAB>(d, ld, J, q % N, N, tab, twfx, C, S);
 #pragma unroll
         for (int u = 0; u < FT; ++u) {
-          const int f = g0 + s * FT + u, e = sc.S[f] - (kDftBits - kDftLow);
+          const int f = g0 + s * FT + u, e = sc.S[f] - kDftUnit;
           const int4 v0 = d[u * ld];
           const long long x0 = ((long long)v0.x << kDftLow) + v0.y, xh = ((long long)v0.z << kDftLow) + v0.w;
-          const w96 re = w_add(C[u], w_shl64(x0 + (q & 1 ? -xh : xh), kDftBits - kDftLow));
+          const w96 re = w_add(C[u], w_shl64(x0 + (q & 1 ? -xh : xh), kDftUnit));
           const bool bad = sc.key[f] >= kNonFinite;
           block[(long)q * sq + f] =
               bad ? make_double2(nan, nan) : make_double2(wj * f64_of_w(re, e), wj * f64_of_w(S[u], e));

@@ -1,4 +1,4 @@
-// 96-bit integers and 28-bit limb pairs: the arithmetic of the FP64 plans' row
+// 96-bit integers and limb pairs: the arithmetic of the FP64 plans' row
 // transforms (rows_w.cuh), built from 32-bit additions with carry and 32 x 32 ->
 // 64-bit multiply-adds.  GB300 executes those at up to 64 times the rate of its
 // FP64 pipe.
