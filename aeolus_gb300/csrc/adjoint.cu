@@ -104,13 +104,13 @@ struct SweAdjDerive {
 };
 
 // The same for the split path: seven contracted forward fields (SweDerive7;
-// the synthesis epilogue forms eta_lam and phi_lam) and the four adjoint ones,
-// the forward fields in double-float arithmetic as in the forward chains.
-// Slicing 29.7 -> 25.8 us at 8 members, l_max 127 (the FP64 derivation bound it);
-// the synthesis has one data tile in seven less.
+// the synthesis epilogue forms eta_lam and phi_lam) and the four adjoint ones.
+// The fields are derived in FP64: the products of the VJP cancel, and deriving
+// them in double-float as the forward chains do raised its zeta errors by 0.9 to
+// 2.6 % and saved nothing (gradient through 8 steps of 8 members, l_max 127: 13.1
+// ms either way).
 struct SweAdjDerive11 {
   static constexpr int NF = 11, NBLK = 13;
-  static constexpr bool kColumnDf = true;
   __host__ __device__ static constexpr int blk(int f) { return f < 7 ? SweDerive7::blk(f) : f + 2; }
   __host__ __device__ static constexpr int lam_blk(int f) { return f < 7 ? SweDerive7::lam_blk(f) : -1; }
   SweAdjDerive d13;
@@ -118,13 +118,6 @@ struct SweAdjDerive11 {
   __device__ void column(int b, int l, int m, double2* v) const {
     SweDerive7{d13.fwd}.column(b, l, m, v);
     d13.adjoint_column(b, l, m, v + 7);
-  }
-  __device__ void column_df(int b, int l, int m, df2* v) const {
-    SweDerive7{d13.fwd}.column_df(b, l, m, v);
-    double2 q[4];
-    d13.adjoint_column(b, l, m, q);
-#pragma unroll
-    for (int f = 0; f < 4; ++f) v[7 + f] = df2_of_f64x2(q[f]);
   }
 };
 
