@@ -482,24 +482,33 @@ def swe_rk4_adjoint(plan_id: int, radius: float, omega: float, gravity: float, m
     return yb.reshape(lead + (3,) + _spec_shape(p.lmax))
 
 
-def swe_rk4_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
-                   state: torch.Tensor, dt: float, forcing: torch.Tensor | None = None,
-                   step: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
-    """(step output or None without `step`, inputs of stages 2 to 4 as
-    [3, B, 3, L+1, L+1]) of one RK4 step from `state`."""
+@torch.library.custom_op("aeolus::swe_rk4_stages", mutates_args=())
+def _swe_rk4_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
+                    state: torch.Tensor, dt: float, forcing: torch.Tensor | None,
+                    step: bool) -> tuple[torch.Tensor, torch.Tensor]:
     p = _PLANS[plan_id]
     s, lead = _flat_spec(state, p.lmax, 3)
     B = s.shape[0]
-    nxt = torch.empty_like(s) if step else None
+    nxt = torch.empty_like(s if step else s[:0])
     stages = torch.empty((3,) + tuple(s.shape), dtype=s.dtype, device=s.device)
     if B:
         w = p.workspace(_lib.OP_SWE_RK4, B)
         prm = _swe_params(radius, omega, gravity, mean_depth, nu4, forcing, p.lmax, s.device)
         check(_lib.load().aeolus_swe_rk4_stages(p.handle, byref(prm), _ptr(s), _ptr(nxt) if step else None,
                                                 _ptr(stages), B, float(dt), _ptr(w), w.numel(), _stream(s.device)))
-    return nxt.reshape(lead + (3,) + _spec_shape(p.lmax)) if step else None, stages
+    return nxt.reshape(lead + (3,) + _spec_shape(p.lmax)) if step else nxt, stages
 
 
+def swe_rk4_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
+                   state: torch.Tensor, dt: float, forcing: torch.Tensor | None = None,
+                   step: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
+    """(step output or None without `step`, inputs of stages 2 to 4 as
+    [3, B, 3, L+1, L+1]) of one RK4 step from `state`."""
+    nxt, stages = _swe_rk4_stages(plan_id, radius, omega, gravity, mean_depth, nu4, state, dt, forcing, step)
+    return nxt if step else None, stages
+
+
+@torch.library.custom_op("aeolus::swe_rk4_adjoint_stages", mutates_args=())
 def swe_rk4_adjoint_stages(plan_id: int, radius: float, omega: float, gravity: float, mean_depth: float, nu4: float,
                            state: torch.Tensor, stages: torch.Tensor, state_bar: torch.Tensor, dt: float,
                            forcing: torch.Tensor | None = None) -> torch.Tensor:
