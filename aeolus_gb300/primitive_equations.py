@@ -234,9 +234,11 @@ class PrimitiveEquationsModel:
 
         y = torch.as_tensor(coeffs).to(torch.complex128).contiguous()
         K, n = self.nlev, self.l_max + 1
-        if stage_validator is None and y.is_cuda and tuple(y.shape[-3:]) == (3 * K + 1, n, n) and y.numel():
+        own = type(self).tendency is PrimitiveEquationsModel.tendency and "tendency" not in vars(self)
+        if own and stage_validator is None and y.is_cuda and tuple(y.shape[-3:]) == (3 * K + 1, n, n) and y.numel():
             # all stages in one library call: the generic step's operations
-            # and roundings on the same tendencies
+            # and roundings on the same tendencies (a model with a tendency of
+            # its own takes the generic step)
             y = y.clone()
             B = y.numel() // ((3 * K + 1) * n * n)
             if nsteps > 0:
