@@ -44,6 +44,14 @@ def _stage_steps(m, y, every):
     return min(every, m._plan.workspace_bytes(_lib.OP_SWE_RK4_ADJOINT, members) // (3 * 16 * y.numel()))
 
 
+def _keeps_stages(model):
+    """Whether the model's steps are the library's: a model that steps by a
+    method of its own keeps nothing, every step goes through that method."""
+    from .shallow_water import ShallowWaterModel
+
+    return getattr(type(model), "rk4", None) is ShallowWaterModel.rk4 and "rk4" not in vars(model)
+
+
 def _swe_segment(m, y, dt, n, keep, last):
     """[(input, stage inputs or None)] of n steps from y, and with `last` the
     state after them."""
@@ -69,7 +77,8 @@ class _SweRk4Checkpointed(torch.autograd.Function):
         y = y0.detach()
         # the backward starts with the last segment: its steps keep their
         # inputs from here on instead of being run again
-        head = (nsteps - 1) // every * every if ctx.needs_input_grad[0] and nsteps > 0 else nsteps
+        keep = ctx.needs_input_grad[0] and _keeps_stages(model)
+        head = (nsteps - 1) // every * every if keep and nsteps > 0 else nsteps
         for i in range(head):
             if i % every == 0:
                 ckpts.append(y.clone())
@@ -87,10 +96,11 @@ class _SweRk4Checkpointed(torch.autograd.Function):
         m = ctx.model
         yb = ybar.contiguous()
         for seg in range(len(ctx.ckpts) - 1, -1, -1):
-            if seg == len(ctx.ckpts) - 1:
+            if seg == len(ctx.ckpts) - 1 and ctx.tail:
                 steps = list(ctx.tail)
             else:
-                steps, _ = _swe_segment(m, ctx.ckpts[seg], ctx.dt, ctx.every, ctx.keep, False)
+                n = min(ctx.every, ctx.nsteps - seg * ctx.every)
+                steps, _ = _swe_segment(m, ctx.ckpts[seg], ctx.dt, n, ctx.keep, False)
             while steps:
                 y, stages = steps.pop()
                 if stages is None:
