@@ -938,7 +938,8 @@ int pe_chain_check(aeolus_plan plan, const aeolus_pe_params* prm, int nlev, cons
   if (int s = pe_check(prm)) return s;
   if (int s = make_sigma(interfaces, nlev, sg)) return s;
   if (batch > 0 && !phi_s) return fail(AEOLUS_ERR_ARG, std::string(who) + ": NULL phi_s");
-  if ((long)batch * (nlev + 1) > 65535)
+  // a Gauss plan's kernels take a level of a member per grid row
+  if (plan->kind == kGauss && (long)batch * (nlev + 1) > 65535)
     return fail(AEOLUS_ERR_ARG, std::string(who) + ": batch (nlev + 1) above 65535");
   return AEOLUS_OK;
 }

@@ -268,7 +268,8 @@ int aeolus_pe_spectral(int lmax, const aeolus_pe_params* params, int nlev, const
  * [L+1], phi_s [L+1][L+1], device; `interfaces` host.  aeolus_pe_rk4 advances
  * `state` in place by nsteps classical steps, the operations and roundings of
  * aeolus_rk4_stage on these tendencies.  Workspace sizes (either pointer may
- * be NULL) from aeolus_pe_workspace_bytes; batch (K + 1) is at most 65535. */
+ * be NULL) from aeolus_pe_workspace_bytes; batch is at most 65535, and on a
+ * Gauss plan batch (K + 1). */
 int aeolus_pe_workspace_bytes(aeolus_plan plan, int nlev, int batch, size_t* tendency_bytes, size_t* rk4_bytes);
 int aeolus_pe_tendency(aeolus_plan plan, const aeolus_pe_params* params, int nlev, const double* interfaces,
                        const double* state, const double* phi_s, double* tendency, int batch, void* work,
