@@ -17,10 +17,15 @@ kernels.  Every backward is a call into ``libaeolus_gb300.so``:
   keeps the stage inputs of a segment too, as long as they fit into the size
   of one step adjoint's workspace (``aeolus_swe_rk4_adjoint_stages``; beyond
   that the step adjoint recomputes them), and the last segment, with which the
-  backward starts, from the forward pass.
+  backward starts, from the forward pass until the backward has used it.
+  ``keep_stages=False`` keeps neither, and neither is kept where the device's
+  memory does not hold them; the gradient is the same bit for bit.
 
-Peak device memory is therefore (checkpoints + two segments) states plus
-three RK4-adjoint workspaces at most, independent of ``nsteps``.
+Peak device memory is therefore (checkpoints + one segment) states plus two
+RK4-adjoint workspaces, of which the graph holds one segment and at most one
+workspace until its backward, independent of ``nsteps``; without kept stages
+(checkpoints + one segment) states plus one workspace, and the graph holds the
+checkpoints alone.
 """
 from __future__ import annotations
 
@@ -70,44 +75,63 @@ def _swe_segment(m, y, dt, n, keep, last):
 
 class _SweRk4Checkpointed(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, y0, model, dt, nsteps, every):
+    def forward(ctx, y0, model, dt, nsteps, every, keep):
         every = max(1, int(every))
         nsteps = int(nsteps)
         ckpts = []
         y = y0.detach()
         # the backward starts with the last segment: its steps keep their
         # inputs from here on instead of being run again
-        keep = ctx.needs_input_grad[0] and _keeps_stages(model)
         head = (nsteps - 1) // every * every if keep and nsteps > 0 else nsteps
-        for i in range(head):
+        tail, keep = None, 0
+        for i in range(nsteps):
             if i % every == 0:
                 ckpts.append(y.clone())
-            y = model.rk4(y, dt, 1, check=False)
-        ctx.keep, ctx.tail = 0, []
-        if head < nsteps:
-            ckpts.append(y.clone())
-            ctx.keep = _stage_steps(model, y, every)
-            ctx.tail, y = _swe_segment(model, ckpts[-1], float(dt), nsteps - head, ctx.keep, True)
+            if i == head:
+                keep = _stage_steps(model, y, every)
+                try:
+                    tail, out = _swe_segment(model, ckpts[-1], float(dt), nsteps - head, keep, True)
+                    break
+                except torch.cuda.OutOfMemoryError:
+                    keep = 0
+            y = out = model.rk4(y, dt, 1, check=False)
         ctx.model, ctx.dt, ctx.nsteps, ctx.every, ctx.ckpts = model, float(dt), nsteps, every, ckpts
-        return y
+        ctx.keep, ctx.tail = keep, tail
+        return out if nsteps > 0 else y
 
     @staticmethod
     def backward(ctx, ybar):
         m = ctx.model
         yb = ybar.contiguous()
         for seg in range(len(ctx.ckpts) - 1, -1, -1):
-            if seg == len(ctx.ckpts) - 1 and ctx.tail:
-                steps = list(ctx.tail)
-            else:
-                n = min(ctx.every, ctx.nsteps - seg * ctx.every)
-                steps, _ = _swe_segment(m, ctx.ckpts[seg], ctx.dt, n, ctx.keep, False)
+            n = min(ctx.every, ctx.nsteps - seg * ctx.every)
+            steps = None
+            if seg == len(ctx.ckpts) - 1:  # kept once: a second backward runs the segment again
+                steps, ctx.tail = ctx.tail, None
+            if steps is None:
+                steps = _rerun(ctx, seg, n)
             while steps:
                 y, stages = steps.pop()
-                if stages is None:
-                    yb = swe_rk4_adjoint(*_swe_args(m), y, yb, ctx.dt, m.forcing)
-                else:
-                    yb = swe_rk4_adjoint_stages(*_swe_args(m), y, stages, yb, ctx.dt, m.forcing)
-        return yb, None, None, None, None
+                if stages is not None:
+                    try:
+                        yb = swe_rk4_adjoint_stages(*_swe_args(m), y, stages, yb, ctx.dt, m.forcing)
+                        continue
+                    except torch.cuda.OutOfMemoryError:
+                        ctx.keep, stages = 0, None
+                    steps = [(x, None) for x, _ in steps]  # the adjoints do not fit beside the stages
+                yb = swe_rk4_adjoint(*_swe_args(m), y, yb, ctx.dt, m.forcing)
+        return yb, None, None, None, None, None
+
+
+def _rerun(ctx, seg, n):
+    """The steps of segment `seg` from its checkpoint."""
+    try:
+        return _swe_segment(ctx.model, ctx.ckpts[seg], ctx.dt, n, ctx.keep, False)[0]
+    except torch.cuda.OutOfMemoryError:
+        if ctx.keep == 0:
+            raise
+        ctx.keep = 0
+    return _swe_segment(ctx.model, ctx.ckpts[seg], ctx.dt, n, 0, False)[0]
 
 
 class _BveRk4Checkpointed(torch.autograd.Function):
@@ -138,11 +162,15 @@ class _BveRk4Checkpointed(torch.autograd.Function):
         return zb, None, None, None, None
 
 
-def swe_rk4_checkpointed(model, y0: torch.Tensor, dt: float, nsteps: int, every: int = 8) -> torch.Tensor:
+def swe_rk4_checkpointed(model, y0: torch.Tensor, dt: float, nsteps: int, every: int = 8, *,
+                         keep_stages: bool = True) -> torch.Tensor:
     """``nsteps`` SWE RK4 steps of ``[..., 3, L+1, L+1]`` states, differentiable
     in ``y0`` through the hand-written adjoint with checkpoints every
-    ``every`` steps (run/engine.py:406-431 differentiated)."""
-    return _SweRk4Checkpointed.apply(y0, model, float(dt), int(nsteps), int(every))
+    ``every`` steps (run/engine.py:406-431 differentiated).  ``keep_stages``
+    trades memory for time (module docstring); without a gradient to come
+    nothing is kept."""
+    keep = bool(keep_stages) and torch.is_grad_enabled() and y0.requires_grad and _keeps_stages(model)
+    return _SweRk4Checkpointed.apply(y0, model, float(dt), int(nsteps), int(every), keep)
 
 
 def bve_rk4_checkpointed(model, z0: torch.Tensor, dt: float, nsteps: int, every: int = 8) -> torch.Tensor:
