@@ -22,8 +22,10 @@ int cuda_check(cudaError_t e, const char* what);
 #define AE_LAUNCH(what) do { int _s = ::aeolus::cuda_check(cudaGetLastError(), what); if (_s) return _s; } while (0)
 
 // ---------------------------------------- programmatic dependent launch
-// The stage kernels of every chain are launched with programmatic stream
-// serialisation: as the CTAs of the previous kernel in the stream exit, this
+// The stage kernels of the Gauss chains, of the primitive equations and of FP64
+// point sets are launched with programmatic stream serialisation (the dense split
+// products of point sets and the finishing kernels of adjoints and vector operators
+// are plain launches): as the CTAs of the previous kernel in the stream exit, this
 // kernel's CTAs take their places, set themselves up (the tensor-core kernels'
 // barriers and TMEM) and wait (griddepcontrol.wait) for the previous grid to
 // complete, with its memory visible, before they touch global memory that it

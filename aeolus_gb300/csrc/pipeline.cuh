@@ -35,11 +35,6 @@ inline int allow_smem(K kern, size_t bytes) {
   return allow_smem_raw(reinterpret_cast<const void*>(kern), bytes);
 }
 
-inline int round_threads(long items, int lo, int hi) {
-  long t = (items + 31) / 32 * 32;
-  return (int)std::max<long>(lo, std::min<long>(hi, t));
-}
-
 // Launch shapes of the three Gauss stages (the autotuner's knobs are the
 // plan's tune_* fields; 0 keeps the built-in heuristic).
 struct LegCfg {

@@ -530,7 +530,7 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
 //  * the digit reversal of the in-place DIT input is arithmetic:
 //    natural index q = 64 t0 + 8 t1 + t2 sits at t0 + R0 (t1 + 8 t2).
 constexpr int kFx8Threads = 128;
-// Threads of a row CTA where the rows are too few to fill the SMs (row_threads_split).
+// Threads of a row CTA where the rows are too few to fill the SMs (split_few_rows).
 constexpr int kFewRowThreads = 320;
 
 template <int R0>
