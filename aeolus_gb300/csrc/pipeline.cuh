@@ -58,12 +58,16 @@ inline int leg_warps(int warps) {
 }
 
 // CTAs that share one (order pair, member chunk) of `warps` warps of items:
-// six CTAs per SM even out the last wave (8 members at l_max 127: 512 pairs
-// on 152 SMs are 4 rounds for 3.4 of work); no CTA gets fewer than two warps,
-// and its share of the columns' derivation stays a few percent.
+// enough for six CTAs per SM, which even out the last wave (24 members at l_max
+// 127 4306 us a step against 4443 with three to five, 8 members 1542 against 1517
+// to 1542), and none with fewer than four warps: each repeats the derivation or the
+// folding of the whole pair.  Against two warps at least: 423 -> 364 us for 4
+// members at l_max 85, 533 -> 507 for 2 at 127, 563 -> 533 for 8 at 63, but 138 ->
+// 142 for one at 42 and 226 -> 238 for 2 at 85; against eight: 246 -> 193 us for
+// one at 85, 308 -> 341 for one at 127.
 inline int leg_shares(const aeolus_plan_impl* p, long ctas, int warps) {
   const long want = (6L * p->sm_count + ctas - 1) / std::max(ctas, 1L);
-  return (int)std::max(1L, std::min<long>(want, warps / 2));
+  return (int)std::max(1L, std::min<long>(want, warps / 4));
 }
 
 template <class Derive>
