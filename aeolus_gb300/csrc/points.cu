@@ -73,16 +73,10 @@ void synth_pass(long M, int K, int N, const double* B, const double* V, double* 
   launch_pdl(points_synth_kernel<NT>, dim3((unsigned)grid), dim3(kPtThreads), 0, st, M, K, N, B, V, out);
 }
 
-// Four basis columns per CTA share each point's data values once there are
-// enough columns to fill the chip that way (four CTAs on each SM); one per
-// CTA below that.
 template <int NT>
-void analysis_pass(int M, long K, int N, const double* B, const double* W, double* C, int sm_count, cudaStream_t st) {
-  const long passes = (N + NT - 1) / NT;
-  if (M >= 16 * sm_count)
-    launch_pdl(points_analysis_kernel<NT, 4>, dim3((unsigned)((M + 3) / 4 * passes)), dim3(kPtThreads), 0, st, M, K, N, B, W, C);
-  else
-    launch_pdl(points_analysis_kernel<NT, 1>, dim3((unsigned)(M * passes)), dim3(kPtThreads), 0, st, M, K, N, B, W, C);
+void analysis_pass(int M, long K, int N, const double* B, const double* W, double* C, cudaStream_t st) {
+  const long grid = M * (long)((N + NT - 1) / NT);
+  launch_pdl(points_analysis_kernel<NT>, dim3((unsigned)grid), dim3(kPtThreads), 0, st, M, K, N, B, W, C);
 }
 
 inline int pass_columns(int N) {
@@ -113,7 +107,7 @@ int points_gemm_synth(const aeolus_plan_impl* p, const double* V, double* out, i
 
 int points_gemm_analysis(const aeolus_plan_impl* p, const double* W, double* C, int ncols, cudaStream_t st) {
   ProfScope prof("points_analysis_f64", st);
-  AE_PT_PASS(analysis_pass, pass_columns(ncols), p->ncol, p->npoints, ncols, p->basis, W, C, p->sm_count, st)
+  AE_PT_PASS(analysis_pass, pass_columns(ncols), p->ncol, p->npoints, ncols, p->basis, W, C, st)
   AE_LAUNCH("points_analysis_kernel");
   return AEOLUS_OK;
 }

@@ -161,56 +161,48 @@ __global__ void __launch_bounds__(kPtThreads) points_synth_kernel(long M, int K,
   }
 }
 
-// C[n * M + c] = sum_p B[c * K + p] W[n * K + p]: CT basis columns per CTA,
-// its threads stride over the points (contiguous in B and W).
-template <int NT, int CT>
+// C[n * M + c] = sum_p B[c * K + p] W[n * K + p]: one basis column per CTA, its
+// threads stride over the points (contiguous in B and W).  Four basis columns per
+// CTA, which share each point's data values, are slower or equal: 40,962 points,
+// 2,809 columns and 8 data columns 1,664 against 1,588 us, 6,561 and 8 3,643
+// against 3,653, 6,561 and 32 14,515 against 14,334.
+template <int NT>
 __global__ void __launch_bounds__(kPtThreads) points_analysis_kernel(int M, long K, int N, const double* __restrict__ B,
                                                                      const double* __restrict__ W,
                                                                      double* __restrict__ C) {
   pdl_wait();
-  __shared__ double sR[kPtThreads / 32][CT * NT];
-  const unsigned cb = (unsigned)((M + CT - 1) / CT);
-  const int n0 = (int)(blockIdx.x / cb) * NT, nn = min(NT, N - n0);
-  const int c0 = (int)(blockIdx.x % cb) * CT;
-  const double* Bc[CT];
+  __shared__ double sR[kPtThreads / 32][NT];
+  const int n0 = (int)(blockIdx.x / (unsigned)M) * NT, nn = min(NT, N - n0);
+  const int c = (int)(blockIdx.x % (unsigned)M);
+  const double* Bc = B + (long)c * K;
   const double* Wn[NT];
 #pragma unroll
-  for (int i = 0; i < CT; ++i) Bc[i] = B + (long)min(c0 + i, M - 1) * K;
-#pragma unroll
   for (int q = 0; q < NT; ++q) Wn[q] = W + (long)(n0 + min(q, nn - 1)) * K;
-  double acc[CT][NT];
+  double acc[NT];
 #pragma unroll
-  for (int i = 0; i < CT; ++i)
-#pragma unroll
-    for (int q = 0; q < NT; ++q) acc[i][q] = 0.0;
+  for (int q = 0; q < NT; ++q) acc[q] = 0.0;
 #pragma unroll 2
   for (long p = threadIdx.x; p < K; p += kPtThreads) {
-    double b[CT], w[NT];
-#pragma unroll
-    for (int i = 0; i < CT; ++i) b[i] = __ldg(Bc[i] + p);
+    const double b = __ldg(Bc + p);
+    double w[NT];
 #pragma unroll
     for (int q = 0; q < NT; ++q) w[q] = __ldcg(Wn[q] + p);
 #pragma unroll
-    for (int i = 0; i < CT; ++i)
-#pragma unroll
-      for (int q = 0; q < NT; ++q) acc[i][q] = fma(b[i], w[q], acc[i][q]);
+    for (int q = 0; q < NT; ++q) acc[q] = fma(b, w[q], acc[q]);
   }
 #pragma unroll
-  for (int i = 0; i < CT; ++i)
-#pragma unroll
-    for (int q = 0; q < NT; ++q) {
-      double v = acc[i][q];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if ((threadIdx.x & 31) == 0) sR[threadIdx.x >> 5][i * NT + q] = v;
-    }
+  for (int q = 0; q < NT; ++q) {
+    double v = acc[q];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sR[threadIdx.x >> 5][q] = v;
+  }
   __syncthreads();
-  for (int e = threadIdx.x; e < CT * NT; e += kPtThreads) {
-    const int i = e / NT, q = e % NT;
-    if (q >= nn || c0 + i >= M) continue;
+  if (threadIdx.x < nn) {
+    const int q = threadIdx.x;
     double v = 0.0;
 #pragma unroll
-    for (int w = 0; w < kPtThreads / 32; ++w) v += sR[w][e];
-    C[(long)(n0 + q) * M + c0 + i] = v;
+    for (int w = 0; w < kPtThreads / 32; ++w) v += sR[w][q];
+    C[(long)(n0 + q) * M + c] = v;
   }
 }
 
