@@ -19,6 +19,9 @@
 //   aeolus_pe_spectral  spectral: 2/3 cuts, Simmons-Burridge geopotential of
 //                       the spectral T, -lap(KE + Phi), l = 0 rows of the
 //                       momentum tendencies pinned.
+//
+// These calls are the C ABI's pieces and the yardstick of the chain's tests; the
+// package runs the whole tendency as one chain (aeolus_pe_tendency, below).
 #include <type_traits>
 
 #include "models.cuh"
@@ -469,7 +472,7 @@ __global__ void pe_spectral_kernel(PeSigma sg, int L, double R, double r_dry, in
 // calls (10 K + 2 fields synthesised, 6 K + 1 analysed to l_max + 1, FP64 grids
 // between the kernels, 14 launches through Python): one FP64 RK4 step at 64 x
 // 128, l_max 42, 8 levels 1.45 -> 0.27 ms; the split tendency of 4 members at
-// 192 x 384, l_max 127, 20 levels 2.13 -> 1.35 ms (columns 376 -> 262 us, bound
+// 192 x 384, l_max 127, 20 levels 2.13 -> 1.26 ms (columns 376 -> 265 us, bound
 // by instruction issue; 110 us of it are the DRAM bytes).
 constexpr int kPeGrid = 9;  // U, V, zeta, delta, T, T_lam, T_snt, eta_lam, eta_snt
 constexpr int kPeProd = 6;  // the four integrands of kPeOutFields, Z_east / cos, Z_north / cos

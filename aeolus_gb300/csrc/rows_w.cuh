@@ -26,7 +26,7 @@
 //
 // Row stage per RK4 stage against FP64 transforms and sums: 8 members at 192 x
 // 384, l_max 127 367 -> 124 us; 3 members on 95 x 190 points, l_max 63 (direct
-// sums) 238 -> 37 us; one member at 128 x 256, l_max 85 28.9 -> 23.9 us (128
+// sums) 238 -> 39 us; one member at 128 x 256, l_max 85 28.9 -> 23.9 us (128
 // CTAs, bound by the latency of one row); 82 fields on 64 x 128 points (grid
 // output) 66 -> 17 us.  Bound by instruction issue (42 k warp instructions per
 // 9 + 4 field row at n = 192; 38 % issue-active at 14 warps per SM, which the

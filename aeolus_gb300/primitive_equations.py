@@ -191,6 +191,8 @@ class PrimitiveEquationsModel:
         self._sigma_host = np.ascontiguousarray(sigma.interfaces_array())
 
     def _ext_plan(self):
+        """The one-degree-extended plan of the separate weak-form curl/div call
+        (the chain needs none)."""
         return self.so._extended_plan()
 
     def _workspace(self, batch: int, rk4: int, device) -> torch.Tensor:
