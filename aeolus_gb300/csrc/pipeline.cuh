@@ -146,7 +146,7 @@ inline void row_args(const aeolus_plan_impl* p, RowArgs& a) {
 
 template <class Pw, int IN_MODE, int OUT_MODE, class FFT>
 int launch_rows_fx(const aeolus_plan_impl* p, const Pw& pw, const RowArgs& a, cudaStream_t st) {
-  const size_t sm = row_fx_smem_bytes<Pw>(p->fftx);
+  const size_t sm = row_fx_smem_bytes<Pw>(p->fftx, p->lmax);
   auto kern = row_kernel_fx<Pw, IN_MODE, OUT_MODE, FFT>;
   int s = allow_smem(kern, sm);
   if (s) return s;
@@ -237,7 +237,7 @@ size_t split_row_smem_bytes(const aeolus_plan_impl* p) {
     case kRowsPfa64: return row_pfa_smem_bytes<Pw, Pfa64>();
     case kRowsPfa32: return row_pfa_smem_bytes<Pw, Pfa32>();
     case kRowsFx8R2: return row_fx8_smem_bytes<Pw>(2);
-    default: return row_fx_smem_bytes<Pw>(p->fftx);
+    default: return row_fx_smem_bytes<Pw>(p->fftx, p->lmax);
   }
 }
 

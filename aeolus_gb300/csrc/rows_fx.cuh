@@ -295,6 +295,10 @@ struct FftFixed {
   }
 };
 
+// Slots of a field's row: its n complex values, and where the direct DFT stages
+// the spectra every order, of which a row too short for its l_max has more.
+__host__ __device__ inline int row_fx_stride(bool use_fft, int n, int L) { return (use_fft || n > L ? n : L) + 1; }
+
 template <class Pw, int IN_MODE, int OUT_MODE, class FFT = FftRuntime>
 __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, const FxW* __restrict__ twfx,
                                             const float4* __restrict__ twdf, const FxConst& kc, int bx, int by) {
@@ -311,8 +315,8 @@ __device__ __forceinline__ void row_fx_body(const RowArgs& a, const Pw& pw, cons
   const int j = bx, b = by;
   const int N = a.fft.N, n = a.fft.n, L = a.L;
   const int ldm = L + 1;
-  const int ns = n + 1;  // padded field stride of the smem rows (see row_body)
   const bool use_fft = FFT::kFixed || a.fft.use_fft != 0;
+  const int ns = row_fx_stride(use_fft, n, L);  // padded field stride of the smem rows
   const int hb = min(52, 56 - (32 - __clz(max(n - 1, 1))));  // |fixed-point FFT input| < 2^hb
   cfx* buf0 = smem_fx;                 // the rows (all in-place FFT work)
   cfx* buf1 = smem_fx + (long)NF * ns;  // staged spectra of the direct DFT (allocated only then)
@@ -807,9 +811,9 @@ constexpr size_t row_fx8_smem_bytes(int R0) {
 // Dynamic shared memory of row_kernel_fx: one row buffer for the in-place
 // FFTs, a second one for the staged spectra of the direct DFT.
 template <class Pw>
-inline size_t row_fx_smem_bytes(const FftInfo& f) {
+inline size_t row_fx_smem_bytes(const FftInfo& f, int L) {
   constexpr int NF = Pw::NIN > Pw::NOUT ? Pw::NIN : Pw::NOUT;
-  return (size_t)(f.use_fft ? 1 : 2) * NF * (f.n + 1) * sizeof(cfx);
+  return (size_t)(f.use_fft ? 1 : 2) * NF * row_fx_stride(f.use_fft != 0, f.n, L) * sizeof(cfx);
 }
 
 template <class Pw, int IN_MODE, int OUT_MODE, class FFT>
